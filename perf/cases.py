@@ -3,7 +3,8 @@ layer and a whole prefill, each through its public entry point.
 
 ``listed()`` names the cases, ``draw(rng)`` gives further ones of the same ranges, ``prepare`` makes what a program holds
 before the call (activations, packed weights, a module or a model), ``run`` is one call, ``work`` the bytes and operations
-that call cannot do without and ``tolerance`` how far two correct implementations of the same precision may be apart.
+that call cannot do without, ``tolerance`` how far two correct implementations of the same precision may be apart and
+``exact`` what plain torch gives for the same inputs in 64 bits.
 
 Kinds:
   layer     ``linear_forward(use_hadamard=True)``, no workspaces: the functional form of the W4A4 linear
@@ -192,3 +193,64 @@ def tolerance(case: dict):
     if kind == "prefill":
         return {"rel": 3e-2}
     return {"rel": 1e-2, "max": 0.5}
+
+
+# ------------------------------------------------------------------------------------------------ the same in 64 bits
+def _transform64(x: torch.Tensor, block: int, scale: float) -> torch.Tensor:
+    """The block transform of bf16 rows with sums in float64, rounded once to bf16 (a rounding point of the format)."""
+    h = x.double().view(x.size(0), -1, block)
+    half = 1
+    while half < block:
+        h = h.view(x.size(0), -1, 2, half)
+        h = torch.stack((h[:, :, 0] + h[:, :, 1], h[:, :, 0] - h[:, :, 1]), dim=2)
+        half *= 2
+    return (h.reshape(x.shape) * scale).to(torch.bfloat16)
+
+
+def _codes64(x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """(codes as float64 [rows, K], scale in float64 [rows, 1]); the codes are taken with the scale rounded to bf16."""
+    x = x.double()
+    s = x.square().mean(dim=1, keepdim=True).sqrt() * (2.513930578568423 * 2 / 15) + 1e-8
+    return (x / s.to(torch.bfloat16).double()).floor().clamp(-8, 7), s
+
+
+def _pack(codes: torch.Tensor) -> torch.Tensor:
+    c = codes.to(torch.int16).bitwise_and_(15).to(torch.uint8)
+    return c[:, ::2] | (c[:, 1::2] << 4)
+
+
+@torch.inference_mode()
+def exact(case: dict, seed: int):
+    kind = case["kind"]
+    if kind == "prefill":
+        return None
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    if kind == "quantise":
+        x = _activations(case["dist"], case["m"], case["k"], g)
+        packed, scale, sums = [], [], []
+        act = torch.tensor(case["block"] ** -0.5).to(torch.bfloat16).item()
+        for rows in x.split(8192):
+            q, s = _codes64(_transform64(rows, case["block"], act))
+            packed.append(_pack(q)), scale.append(s), sums.append(q.sum(dim=1, keepdim=True).to(torch.int32))
+        return torch.cat(packed), torch.cat(scale), torch.cat(sums)
+    w = (0.02 * torch.randn(case["n"], case["k"], generator=g, device=DEV)).to(torch.bfloat16)
+    x = None if kind == "prepare" else _activations(case["dist"], case["m"], case["k"], g)
+    bias = 0.1 * torch.randn(case["n"], generator=g, device=DEV) if kind == "module" else None
+    if kind != "plain":  # weights carry the fp32 constant, activations its bf16 rounding
+        w = _transform64(w, 128, torch.tensor(128.0).rsqrt().item())
+        x = None if x is None else _transform64(x, 128, torch.tensor(128.0).rsqrt().to(torch.bfloat16).item())
+    qw, sw = _codes64(w)
+    del w
+    if kind == "prepare":
+        return _pack(qw), sw, (qw.sum(dim=1, keepdim=True) + case["k"] // 2).to(torch.int32)
+    qa, sa = _codes64(x)
+    sa, sw = sa.to(torch.bfloat16).double(), sw.to(torch.bfloat16).double()
+    y = torch.empty(case["m"], case["n"], dtype=torch.float64, device=DEV)
+    for i in range(0, case["n"], 4096):  # (a + 1/2) . (w + 1/2) is what the offsets of the integer path add up to
+        y[:, i:i + 4096] = (qa + 0.5) @ (qw[i:i + 4096] + 0.5).T
+    y *= sa
+    y *= sw.T
+    if bias is not None:
+        rows = 3 if case["m"] % 3 == 0 else 1
+        y = (y + bias.to(torch.bfloat16)).view(rows, case["m"] // rows, case["n"])
+    return y
