@@ -273,6 +273,16 @@ int quest_b200_copy_block_to_peers_cuda(const void* src, void* const* dsts, int 
 int hadamard_transform_cuda_bf16(void* out_ptr, const void* x_ptr, int group_size, int batch_size, int block,
                                  int weight_side, cudaStream_t stream);
 
+/*
+ * find_scale_int4 + quantize_int4 (packed codes and row sums) in one pass over x, each row read once; with weight_block
+ * (64, 128 or 256) behind the weight-side Hadamard transform (entries +-fp32(block^-0.5), rounded to bf16), i.e. the whole
+ * of gemm-quest/benchmarks/utils.py:20-53 for a dense weight.  row_sum_add is added to every row sum (K / 2 for w_add).
+ * The same bits as the separate calls.  K must be a multiple of 8 and at most 65536, x and the packed codes 16-byte
+ * aligned (QB200_ERR_UNSUPPORTED otherwise: use the separate calls).
+ */
+int scale_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* scale_ptr, void* x_int_row_sum_ptr, const void* x_ptr,
+                                  int group_size, int batch_size, int weight_block, int row_sum_add, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

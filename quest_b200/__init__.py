@@ -402,6 +402,32 @@ def fused_matmul_dequantize_a8(
     return out
 
 
+def scale_quantize_int4(
+        x: torch.Tensor,
+        weight_block: int = 0,
+        row_sum_add: int = 0,
+        x_int_packed: torch.Tensor = None,
+        scale: torch.Tensor = None,
+        x_int_row_sum: torch.Tensor = None,
+) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """``find_scale_int4`` + ``quantize_int4`` (packed codes, row sums + ``row_sum_add``) in one pass over x [M, K], with
+    ``weight_block`` behind the weight-side Hadamard transform.  The same bits as the separate ops.  Only for what
+    ``one_pass_ok`` accepts.  Returns (x_int_packed, scale, x_int_row_sum)."""
+    assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.is_contiguous()
+    m, k = x.shape
+    x_int_packed, scale, x_int_row_sum = _quant_outputs(m, k, x, x_int_packed, scale, x_int_row_sum)
+    dev = _lib.require_cuda(x, scale, x_int_packed, x_int_row_sum)
+    _call("scale_quantize_int4_cuda_bf16", dev, _lib.ptr(x_int_packed), _lib.ptr(scale), _lib.ptr(x_int_row_sum), _lib.ptr(x),
+          k, m, int(weight_block), int(row_sum_add), _lib.stream_of(x))
+    return x_int_packed, scale, x_int_row_sum
+
+
+def one_pass_ok(x: torch.Tensor, weight_block: int = 0) -> bool:
+    """Whether ``scale_quantize_int4`` takes x: bf16 rows of whole 16-byte pieces that one block can hold."""
+    return (x.dim() == 2 and x.dtype == torch.bfloat16 and x.is_contiguous() and 0 < x.size(1) <= 65536 and x.size(1) % 8 == 0
+            and (weight_block == 0 or weight_block in (64, 128, 256) and x.size(1) % weight_block == 0) and x.data_ptr() % 16 == 0)
+
+
 def hadamard_transform(x: torch.Tensor, block: int = 128, weight_side: bool = False, out: torch.Tensor = None) -> torch.Tensor:
     """bf16(H_block @ x) blockwise along the last dim.  ``weight_side`` selects the exact fp32
     normalisation of gemm-quest/benchmarks/utils.py:39 instead of the bf16 one of utils.py:17."""

@@ -36,6 +36,7 @@ struct RowParams {
     float had_scale;               // Hadamard normalisation constant
     int x_out_mode;                // 0 none, 1 transformed values, 2 dequantised values
     int quantize;                  // 0: stop after the scale (find_scale / transform only)
+    int row_sum_add;               // row_kernel only: constant added to every row sum
 };
 
 constexpr int kUnit = 1024;        // elements per warp-unit
@@ -272,7 +273,7 @@ __global__ void __launch_bounds__(UNITS == 1 ? 256 : 512) row_kernel(const RowPa
         if (threadIdx.x == 0) {
             int tot = 0;
             for (int i = 0; i < nwarps; ++i) tot += red_i[i];
-            p.row_sum[row] = tot >> 4;  // exact: every term is a multiple of 16
+            p.row_sum[row] = (tot >> 4) + p.row_sum_add;  // exact: every term is a multiple of 16
         }
     }
 }
@@ -1148,6 +1149,28 @@ extern "C" int hadamard_transform_cuda_bf16(void* out_ptr, const void* x_ptr, in
     const float exact = (float)(1.0 / sqrt((double)block));  // fp32 rounding of block^-0.5
     p.had_scale = weight_side ? exact : __bfloat162float(__float2bfloat16_rn(exact));
     return run_rows(p, block, true, stream);
+}
+
+extern "C" int scale_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* scale_ptr, void* x_int_row_sum_ptr,
+                                             const void* x_ptr, int group_size, int batch_size, int weight_block,
+                                             int row_sum_add, cudaStream_t stream) {
+    if (group_size < 0 || batch_size < 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (weight_block != 0 && weight_block != 64 && weight_block != 128 && weight_block != 256) return QB200_ERR_UNSUPPORTED;
+    if (batch_size == 0) return QB200_OK;
+    if (!x_int_packed_ptr || !scale_ptr || !x_ptr || group_size == 0) return QB200_ERR_INVALID_ARGUMENT;
+    if ((group_size & 1) || (weight_block != 0 && group_size % weight_block != 0)) return QB200_ERR_INVALID_ARGUMENT;
+    RowParams p{};
+    p.x = static_cast<const __nv_bfloat16*>(x_ptr);
+    p.scale_out = static_cast<__nv_bfloat16*>(scale_ptr);
+    p.q_packed = static_cast<uint8_t*>(x_int_packed_ptr);
+    p.row_sum = static_cast<int32_t*>(x_int_row_sum_ptr);
+    p.row_sum_add = row_sum_add;
+    p.K = group_size;
+    p.M = batch_size;
+    p.quantize = 1;
+    p.had_scale = weight_block != 0 ? (float)(1.0 / sqrt((double)weight_block)) : 1.f;  // weights carry the fp32 constant
+    if (!vector_path_ok(p)) return QB200_ERR_UNSUPPORTED;
+    return run_rows(p, weight_block, false, stream);
 }
 
 extern "C" int add_mul_vv_cuda_bf16(void* mat_d, const void* vec_a_add, const void* vec_a_mul, const void* vec_b_add,

@@ -33,6 +33,10 @@ def preprocess_weight(
     if use_sparse:
         raise NotImplementedError("quest_b200 implements the dense W4A4 path only")
     weight = weight.contiguous()
+    if quest.one_pass_ok(weight, block if use_hadamard else 0):
+        w_int_packed, w_scale, w_add = quest.scale_quantize_int4(weight, weight_block=block if use_hadamard else 0,
+                                                                 row_sum_add=weight.size(1) // 2)
+        return w_int_packed, w_scale, w_add, None
     if use_hadamard:
         weight = quest.hadamard_transform(weight, block=block, weight_side=True)
     N, K = weight.shape
