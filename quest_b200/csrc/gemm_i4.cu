@@ -109,7 +109,6 @@ struct EpilogueParams {
     int slab_ints;          // slab_rows * 256: a slab holds only the rows a tile can have (M rounded up to 8, at most 128)
     int* counters;          // one per output tile, all zero between launches
     int tma_store;          // 256 x 256 kernel, fused: the output tensor map is valid (the last tile leaves as bulk tensor stores)
-    int tma_store16;        // int8-operand variant: the 16-column output map is valid too (earlier tiles leave as small bulk stores)
     int test_skip_producer; // tests only: the TMA producer issues nothing, so that every bounded wait of the launch runs out
     // 256-row kernel: the N range is cut into col_count tile columns whose widths are multiples of 16, at most 256; the
     // first col_rem of them are (col_units + 1) * 16 wide, the others col_units * 16 (col_units = 16, col_rem = 0: all 256)
@@ -243,7 +242,7 @@ gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // them still reaches, so that they leave the tile loop together (none is left waiting at a later named barrier).
     volatile int* epi_abort = reinterpret_cast<volatile int*>(smem_raw + (tmem_slot + 12 - smem_u32(smem_raw)));
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform, and known to be
     const int lane = threadIdx.x & 31;
 
     const int tiles_m = (M + BM - 1) / BM;
@@ -321,37 +320,38 @@ gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
-            uint32_t it = 0, local_tile = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++local_tile) {
-                const uint32_t acc = local_tile & 1u, acc_ph = (local_tile >> 1) & 1u;
-                if (!(ok = mbar_wait(tmem_empty + 8 * acc, acc_ph ^ 1u, 3))) break;
+        // ------------------------------ MMA issuer (all lanes walk the loop, see elect_one) ------------------------
+        const uint64_t desc0 = make_smem_desc(u_base);
+        uint32_t s = 0, ph = 0, local_tile = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++local_tile) {
+            const uint32_t acc = local_tile & 1u, acc_ph = (local_tile >> 1) & 1u;
+            ok = __all_sync(0xffffffffu, mbar_wait(tmem_empty + 8 * acc, acc_ph ^ 1u, 3));
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_acc + acc * BN;
+            const int kb0 = kb_first(item);
+            for (int kb = kb0, kb1 = kb_last(item); kb < kb1 && ok; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full_u + 8 * s, ph, 4));
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_acc + acc * BN;
-                const int kb0 = kb_first(item);
-                for (int kb = kb0, kb1 = kb_last(item); kb < kb1; ++kb, ++it) {
-                    const uint32_t s = it % C::U_STAGES, ph = (it / C::U_STAGES) & 1u;
-                    if (!(ok = mbar_wait(full_u + 8 * s, ph, 4))) break;
-                    tc_fence_after();
-                    if (it == 0) QB_TRACE(1);
-                    const uint32_t a_addr = u_base + s * C::U_BYTES;
-                    const uint32_t b_addr = a_addr + BM * U8_ROW;
+                const uint64_t da = desc0 + (uint64_t)(s * (C::U_BYTES >> 4)), db = da + ((BM * U8_ROW) >> 4);
+                if (elect_one()) {
+                    umma_i8(d_tmem, da, db, C::IDESC, kb != kb0 ? 1u : 0u);
 #pragma unroll
-                    for (int j = 0; j < BK / 32; ++j) {
-                        umma_i8(d_tmem, make_smem_desc(a_addr + 32 * j), make_smem_desc(b_addr + 32 * j), C::IDESC,
-                                (kb != kb0 || j != 0) ? 1u : 0u);
-                    }
+                    for (int j = 1; j < BK / 32; ++j) umma_i8(d_tmem, da + 2 * j, db + 2 * j, C::IDESC, 1u);
                     umma_commit(empty_u + 8 * s);  // frees the int8 stage once these MMAs have read it
                 }
-                if (ok) umma_commit(tmem_full + 8 * acc);
+                __syncwarp();
+                if (++s == C::U_STAGES) s = 0, ph ^= 1u;
             }
-            // Everything issued so far must have completed before tensor memory is released.
-            umma_commit(mma_done);
-            mbar_wait(mma_done, 0, 5);
-            QB_TRACE(2);
+            if (ok && elect_one()) umma_commit(tmem_full + 8 * acc);
+            __syncwarp();
         }
+        // Everything issued so far must have completed before tensor memory is released.
+        if (elect_one()) umma_commit(mma_done);
+        __syncwarp();
+        mbar_wait(mma_done, 0, 5);
+        QB_TRACE(2);
     } else if (warp < kFirstUnpackWarp) {
         // ------------------------------ epilogue ------------------------------
         const int quad = warp & 3;  // tensor-memory lane quadrant this warp may read
@@ -620,8 +620,7 @@ constexpr int kPushWarps = 2, kFirstPush = kFirstUnpack + kUnpackWarps;
 constexpr int kWarps = kFirstPush + kPushWarps;
 constexpr int kThreads = kWarps * 32;
 constexpr int VEC_BYTES = TN * 8;
-constexpr int A_STAGES = 3;  // A8 variant: ring of the int8 A tiles (two in the A halves of the int8 stages, one behind the packed B ring)
-constexpr int NUM_BARS = 2 * P_STAGES + 2 * U_STAGES + 2 + 1 + 4 + 2 * A_STAGES;
+constexpr int NUM_BARS = 2 * P_STAGES + 2 * U_STAGES + 2 + 1 + 4;
 constexpr int LAYOUT_BYTES = U_STAGES * U_BYTES + P_STAGES * P_BYTES + VEC_BYTES + NUM_BARS * 8 + 16;
 constexpr int SMEM_BYTES = 232448;  // all the shared memory one CTA can have; the layout needs a 1024-byte aligned start
 static_assert(LAYOUT_BYTES <= SMEM_BYTES, "layout does not fit");
@@ -690,51 +689,7 @@ __device__ __forceinline__ void wide_convert_columns(const EpilogueParams& ep, c
                                                      const CUtensorMap* peer_maps, int n_peer_maps, uint32_t t_row,
                                                      int row, bool row_ok, int a_add, float half_a_mul, const int* sb_add,
                                                      const float* sb_mul, int n0, int N, int c_begin, int c_end,
-                                                     uint32_t stage_base, int warp_row0, int lane,
-                                                     const CUtensorMap* tmap_d16 = nullptr, uint32_t mini_base = 0,
-                                                     uint32_t* mini_count = nullptr) {
-    if (FUSED && mini_base != 0) {
-        // A tile that is not the CTA's last one (int8-operand variant): the rings belong to the next tile already, but
-        // 16 KB of shared memory are free there - two 1 KB slabs per epilogue warp.  The warp writes 32 rows x 16
-        // columns of bf16 (dense rows of 32 bytes) into one slab while the bulk store of the other is still being
-        // read, so the stores leave through the copy engine behind the arithmetic instead of occupying the warp's store
-        // path (about 3 us per tile), and tensor memory is released for the next tile's MMAs as soon as it has been
-        // read.  Rows and columns outside the matrix are clipped by the tensor map.
-        uint32_t piece = *mini_count;
-#pragma unroll 1
-        for (int c0 = c_begin; c0 < c_end; c0 += 64) {
-            if (n0 + c0 >= N) break;  // warp-uniform
-            uint32_t r0[32], r1[32];
-            tmem_ld32(t_row + c0, r0);
-            tmem_ld32(t_row + c0 + 32, r1);
-            tmem_ld_wait();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (c0 + 32 * h >= c_end) break;  // widths are multiples of 16: a tile may end inside a chunk
-                uint32_t w[16];
-                dequant_chunk(h == 0 ? r0 : r1, a_add, half_a_mul, sb_add + c0 + 32 * h, sb_mul + c0 + 32 * h, w);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const int c = c0 + 32 * h + 16 * q;
-                    if (c >= c_end) break;
-                    const uint32_t slab = mini_base + (piece & 1u) * 1024u;
-                    if (lane == 0) bulk_wait_read_but_one();  // the store that used this slab two pieces ago has read it
-                    __syncwarp();
-                    sts128(slab + lane * 32, make_uint4(w[8 * q], w[8 * q + 1], w[8 * q + 2], w[8 * q + 3]));
-                    sts128(slab + lane * 32 + 16, make_uint4(w[8 * q + 4], w[8 * q + 5], w[8 * q + 6], w[8 * q + 7]));
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        tma_store_2d(tmap_d16, slab, n0 + c, warp_row0);
-                        bulk_commit_group();
-                    }
-                    ++piece;
-                }
-            }
-        }
-        *mini_count = piece;
-        return;
-    }
+                                                     uint32_t stage_base, int warp_row0, int lane) {
 #pragma unroll 1
     for (int cx = c_begin; cx < c_end; cx += 64) {
         // a tile width that is no multiple of 64: the last piece starts earlier and rewrites columns of the one before
@@ -781,14 +736,10 @@ __device__ __forceinline__ void wide_convert_columns(const EpilogueParams& ep, c
 
 // PUSH: the multi-GPU variant (two more warps that copy finished tiles to the peers, helped by the epilogue warps on
 // a CTA's last tile); the single-GPU instantiation carries none of that code and is launched without those warps.
-// A8 (single GPU only): the A operand arrives already as int8 in operand order (see hadamard_quant_tc_kernel<HB, true>):
-// one more warp copies its tiles with TMA (128-byte swizzle) straight into the int8 ring, the unpack warps handle
-// only B, and the main loop is bound by the MMAs instead of the unpack.
-template <bool FUSED, bool PUSH, bool A8 = false, bool CLIP = A8>
-__global__ void __launch_bounds__(PUSH ? wide::kThreads : (A8 ? wide::kThreads - 32 : wide::kThreads - 32 * wide::kPushWarps), 1)
+template <bool FUSED, bool PUSH, bool CLIP>
+__global__ void __launch_bounds__(PUSH ? wide::kThreads : wide::kThreads - 32 * wide::kPushWarps, 1)
 gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                    const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_d16,
-                    const __grid_constant__ PeerMaps<PUSH> peers, const __grid_constant__ EpilogueParams ep, const int M,
+                    const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ PeerMaps<PUSH> peers, const __grid_constant__ EpilogueParams ep, const int M,
                     const int N, const int K) {
     using namespace wide;
     extern __shared__ uint8_t smem_raw[];
@@ -811,16 +762,11 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const uint32_t mma_done = tmem_empty + 8;
     const uint32_t out_ready = mma_done + 8;    // [2]
     const uint32_t push_free = out_ready + 16;  // [2]
-    const uint32_t full_a = push_free + 16;      // [A_STAGES] A8 only
-    const uint32_t empty_a = full_a + 8 * A_STAGES;
-    const uint32_t tmem_slot = empty_a + 8 * A_STAGES;
+    const uint32_t tmem_slot = push_free + 16;
     volatile uint32_t* tmem_slot_ptr = reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - raw_base));
     volatile int* epi_abort = reinterpret_cast<volatile int*>(smem_raw + (tmem_slot + 12 - raw_base));  // see gemm_i4_kernel
-    // A8: packed B stages are compact (TN * 64 bytes each), which leaves room for a third A slot behind them
-    constexpr int PB_BYTES = A8 ? TN * PK_ROW : P_BYTES;
-    auto a_slot = [&](uint32_t sa) { return sa < 2 ? u_base + sa * U_BYTES : p_base + P_STAGES * (TN * PK_ROW); };
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);  // uniform, and known to be
     const int lane = threadIdx.x & 31;
     const int tiles_m = (M + TM - 1) / TM;
     const int num_tiles = tiles_m * ep.col_count;
@@ -837,10 +783,6 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             mbar_init(full_u + 8 * i, kUnpackWarps);
             mbar_init(empty_u + 8 * i, 1);
         }
-        for (int i = 0; i < A_STAGES; ++i) {
-            mbar_init(full_a + 8 * i, 1);
-            mbar_init(empty_a + 8 * i, 1);
-        }
         mbar_init(tmem_full, 1);
         mbar_init(tmem_empty, kEpiWarps);
         mbar_init(mma_done, 1);
@@ -853,17 +795,17 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // The first copies of the CTA's first tile leave before tensor memory is allocated and the CTA has synchronised:
         // they need nothing but the barriers initialised above (this thread is also the producer thread below).
         if (ep.test_skip_producer == 0 && (int)blockIdx.x < num_tiles) {
-            if (!A8) wait_for_preceding_grid();  // these copies include A tiles
-            if (!A8) tma_prefetch_desc(&tmap_a);
+            wait_for_preceding_grid();  // these copies include A tiles
+            tma_prefetch_desc(&tmap_a);
             tma_prefetch_desc(&tmap_b);
             const int m0 = ((int)blockIdx.x % tiles_m) * TM;
             int n0, bn;
             column_range(ep, (int)blockIdx.x / tiles_m, n0, bn);
             for (; pre_issued < (uint32_t)P_STAGES && (int)pre_issued < num_kb; ++pre_issued) {
-                mbar_arrive_expect_tx(full_p + 8 * pre_issued, PB_BYTES);
-                const uint32_t dst = p_base + pre_issued * PB_BYTES;
-                if (!A8) tma_load_2d(dst, &tmap_a, (int)pre_issued * PK_ROW, m0, full_p + 8 * pre_issued);
-                tma_load_2d(A8 ? dst : dst + TM * PK_ROW, &tmap_b, (int)pre_issued * PK_ROW, n0, full_p + 8 * pre_issued);
+                mbar_arrive_expect_tx(full_p + 8 * pre_issued, P_BYTES);
+                const uint32_t dst = p_base + pre_issued * P_BYTES;
+                tma_load_2d(dst, &tmap_a, (int)pre_issued * PK_ROW, m0, full_p + 8 * pre_issued);
+                tma_load_2d(dst + TM * PK_ROW, &tmap_b, (int)pre_issued * PK_ROW, n0, full_p + 8 * pre_issued);
             }
         }
     }
@@ -876,9 +818,7 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tc_fence_after();
     const uint32_t tmem_acc = *tmem_slot_ptr;
     let_dependents_launch();  // only now that tensor memory is allocated (see gemm_i4_kernel)
-    // The packed variants load A from the first copy on: every thread waits here.  A8: only the warps that touch the
-    // quantiser's outputs wait (A producer, epilogue), the weights are requested, copied and unpacked before.
-    if (!A8) wait_for_preceding_grid();
+    wait_for_preceding_grid();  // A is loaded from the first copy on: every thread waits here
 
     if (warp == 0) {
         // ------------------------------ TMA producer ------------------------------
@@ -893,10 +833,10 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     if (it < pre_issued) continue;  // left before the CTA synchronised
                     const uint32_t s = it % P_STAGES, ph = (it / P_STAGES) & 1u;
                     if (!(ok = mbar_wait(empty_p + 8 * s, ph ^ 1u, 1))) break;
-                    mbar_arrive_expect_tx(full_p + 8 * s, PB_BYTES);
-                    const uint32_t dst = p_base + s * PB_BYTES;
-                    if (!A8) tma_load_2d(dst, &tmap_a, kb * PK_ROW, m0, full_p + 8 * s);
-                    tma_load_2d(A8 ? dst : dst + TM * PK_ROW, &tmap_b, kb * PK_ROW, n0, full_p + 8 * s);
+                    mbar_arrive_expect_tx(full_p + 8 * s, P_BYTES);
+                    const uint32_t dst = p_base + s * P_BYTES;
+                    tma_load_2d(dst, &tmap_a, kb * PK_ROW, m0, full_p + 8 * s);
+                    tma_load_2d(dst + TM * PK_ROW, &tmap_b, kb * PK_ROW, n0, full_p + 8 * s);
                 }
             }
             const uint32_t pending = it < (uint32_t)P_STAGES ? it : (uint32_t)P_STAGES;
@@ -906,46 +846,43 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             }
         }
     } else if (warp == 1) {
-        // ------------------------------ MMA issuer ------------------------------
-        if (lane == 0) {
-            uint32_t it = 0, local_tile = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
-                const int m0 = (tile % tiles_m) * TM;
-                const int halves = (m0 + 128 < M) ? 2 : 1;  // the lower accumulator is skipped when its rows are all outside M
-                int n0, bn;
-                column_range(ep, tile / tiles_m, n0, bn);
-                const uint32_t idesc = IDESC_BASE | ((uint32_t)(bn >> 3) << 17);
-                if (!(ok = mbar_wait(tmem_empty, (local_tile & 1u) ^ 1u, 3))) break;
+        // ------------------------------ MMA issuer (all lanes walk the loop, see elect_one) ------------------------
+        const uint64_t desc0 = make_smem_desc(u_base);
+        uint32_t s = 0, ph = 0, local_tile = 0;
+        bool ok = true;
+        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
+            const int m0 = (tile % tiles_m) * TM;
+            const bool both = m0 + 128 < M;  // the lower accumulator is skipped when its rows are all outside M
+            int n0, bn;
+            column_range(ep, tile / tiles_m, n0, bn);
+            const uint32_t idesc = IDESC_BASE | ((uint32_t)(bn >> 3) << 17);
+            ok = __all_sync(0xffffffffu, mbar_wait(tmem_empty, (local_tile & 1u) ^ 1u, 3));
+            tc_fence_after();
+            for (int kb = 0; kb < num_kb && ok; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full_u + 8 * s, ph, 4));
+                if (!ok) break;
                 tc_fence_after();
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const uint32_t s = it % U_STAGES, ph = (it / U_STAGES) & 1u;
-                    if (!(ok = mbar_wait(full_u + 8 * s, ph, 4))) break;
-                    tc_fence_after();
-                    if (it == 0) QB_TRACE(1);
-                    const uint32_t sa = it % A_STAGES;
-                    if (A8) {
-                        if (!(ok = mbar_wait(full_a + 8 * sa, (it / A_STAGES) & 1u, 21))) break;
-                        tc_fence_after();
-                    }
-                    const uint32_t a_addr = A8 ? a_slot(sa) : u_base + s * U_BYTES;
-                    const uint32_t b_addr = u_base + s * U_BYTES + TM * U8_ROW;
+                const uint64_t da = desc0 + (uint64_t)(s * (U_BYTES >> 4)), dl = da + ((128 * U8_ROW) >> 4), db = da + ((TM * U8_ROW) >> 4);
+                if (elect_one()) {
+                    umma_i8(tmem_acc, da, db, idesc, kb != 0 ? 1u : 0u);
+                    if (both) umma_i8(tmem_acc + TN, dl, db, idesc, kb != 0 ? 1u : 0u);
 #pragma unroll
-                    for (int j = 0; j < BK / 32; ++j) {
-                        const uint64_t db = make_smem_desc(b_addr + 32 * j);
-                        umma_i8(tmem_acc, make_smem_desc(a_addr + 32 * j), db, idesc, (kb | j) != 0 ? 1u : 0u);
-                        if (halves == 2)
-                            umma_i8(tmem_acc + TN, make_smem_desc(a_addr + 128 * U8_ROW + 32 * j), db, idesc, (kb | j) != 0 ? 1u : 0u);
+                    for (int j = 1; j < BK / 32; ++j) {
+                        umma_i8(tmem_acc, da + 2 * j, db + 2 * j, idesc, 1u);
+                        if (both) umma_i8(tmem_acc + TN, dl + 2 * j, db + 2 * j, idesc, 1u);
                     }
                     umma_commit(empty_u + 8 * s);
-                    if (A8) umma_commit(empty_a + 8 * sa);
                 }
-                if (ok) umma_commit(tmem_full);
+                __syncwarp();
+                if (++s == U_STAGES) s = 0, ph ^= 1u;
             }
-            umma_commit(mma_done);
-            mbar_wait(mma_done, 0, 5);
-            QB_TRACE(2);
+            if (ok && elect_one()) umma_commit(tmem_full);
+            __syncwarp();
         }
+        if (elect_one()) umma_commit(mma_done);
+        __syncwarp();
+        mbar_wait(mma_done, 0, 5);
+        QB_TRACE(2);
     } else if (warp < kFirstUnpack) {
         // ------------------------------ epilogue ------------------------------
         const int quad = warp & 3;                  // tensor-memory lane quadrant this warp may read
@@ -954,9 +891,8 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         uint8_t* vec_ptr = smem_raw + (vec_base - raw_base);
         int* sb_add = reinterpret_cast<int*>(vec_ptr);
         float* sb_mul = reinterpret_cast<float*>(vec_ptr + TN * 4);
-        uint32_t local_tile = 0, mini_pieces = 0;
+        uint32_t local_tile = 0;
         bool ok = true;
-        if (A8) wait_for_preceding_grid();  // the row sums and scales come from the quantiser
         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local_tile) {
             const int m0 = (tile % tiles_m) * TM;
             int n0, bn;
@@ -991,14 +927,9 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const bool last = tile + (int)gridDim.x >= num_tiles;
             const bool staged = FUSED && last && ep.tma_store;
             const uint32_t stage_base = staged ? u_base + (uint32_t)(half * 4 + quad) * 16384u : 0u;
-            // int8-operand variant, earlier tiles: the 16 KB behind the third A slot hold two 1 KB slabs per epilogue warp
-            const uint32_t mini_base = (A8 && FUSED && !staged && ep.tma_store16)
-                                           ? p_base + (uint32_t)(P_STAGES * (TN * PK_ROW) + TM * U8_ROW) + (uint32_t)(warp - kFirstEpi) * 2048u
-                                           : 0u;
             if (m0 + half * 128 < M)  // warp-uniform: otherwise this accumulator was not computed
                 wide_convert_columns<FUSED>(ep, &tmap_d, peers.m, PUSH ? ep.n_peer : 0, t_row, row, row_ok, a_add, half_a_mul,
-                                            sb_add, sb_mul, n0, N, 0, bn, stage_base, m0 + half * 128 + quad * 32, lane,
-                                            &tmap_d16, mini_base, &mini_pieces);
+                                            sb_add, sb_mul, n0, N, 0, bn, stage_base, m0 + half * 128 + quad * 32, lane);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tmem_empty);
@@ -1015,28 +946,6 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     push_tile_rows(ep, m0, n0, min(TM, M - m0), min(bn, N - n0), kPushWarps + (warp - kFirstEpi),
                                    kPushWarps + kEpiWarps, lane);
                 }
-            }
-        }
-    } else if (A8 && warp == kFirstPush) {
-        // ------------------------------ A operand producer (A8 only; there are no push warps then) -----------
-        if (lane == 0) {
-            tma_prefetch_desc(&tmap_a);
-            wait_for_preceding_grid();  // the A operand is the quantiser's output
-            uint32_t it = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int m0 = (tile % tiles_m) * TM;
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const uint32_t sa = it % A_STAGES, aph = (it / A_STAGES) & 1u;
-                    if (!(ok = mbar_wait(empty_a + 8 * sa, aph ^ 1u, 19))) break;
-                    mbar_arrive_expect_tx(full_a + 8 * sa, TM * U8_ROW);
-                    tma_load_2d(a_slot(sa), &tmap_a, kb * U8_ROW, m0, full_a + 8 * sa);
-                }
-            }
-            const uint32_t pending = it < (uint32_t)A_STAGES ? it : (uint32_t)A_STAGES;
-            for (uint32_t j = 0; j < pending; ++j) {  // do not leave while a copy of ours may still land
-                const uint32_t i2 = it - 1 - j;
-                mbar_wait(full_a + 8 * (i2 % A_STAGES), (i2 / A_STAGES) & 1u, 20);
             }
         }
     } else if (warp >= kFirstPush) {
@@ -1084,11 +993,11 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 ok = mbar_wait(full_p + 8 * ps, pph, 7) && mbar_wait(empty_u + 8 * us, uph ^ 1u, 8);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const uint32_t src = A8 ? p_base + ps * PB_BYTES - TM * PK_ROW : p_base + ps * P_BYTES;  // rows are numbered from the A rows on
+                const uint32_t src = p_base + ps * P_BYTES;
                 const uint32_t dst = u_base + us * U_BYTES;
                 constexpr int ITEMS = (TM + TN) * 4 / (kUnpackWarps * 32);  // 8
 #pragma unroll
-                for (int h = A8 ? 1 : 0; h < 2; ++h) {  // the first half of the items are the A rows
+                for (int h = 0; h < 2; ++h) {  // the first half of the items are the A rows
                     uint4 pk[ITEMS / 2];
 #pragma unroll
                     for (int i = 0; i < ITEMS / 2; ++i) {
@@ -1124,6 +1033,8 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tmem_dealloc(tmem_acc, 512);
     }
 }
+
+#include "gemm_i4_pair.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // Host side
@@ -1307,17 +1218,16 @@ static int encode_output_map(CUtensorMap* map, void* base, long long ld, int M, 
                ? QB200_OK : QB200_ERR_DRIVER;
 }
 
-// The same output as 32-row x 16-column boxes of dense 32-byte rows (no swizzle): what an epilogue warp of the
-// int8-operand variant stores per piece of a tile that is not its CTA's last one.
-static int encode_output_map16(CUtensorMap* map, void* base, long long ld, int M, int N) {
+// ... and as 32-row x 32-column boxes of 64-byte rows, 64-byte swizzle: the pieces of the pair kernel.
+static int encode_output_map32(CUtensorMap* map, void* base, long long ld, int M, int N) {
     EncodeTiledFn fn = get_encode_fn();
     if (fn == nullptr) return QB200_ERR_DRIVER;
     const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {16, 32};
+    const cuuint32_t box[2] = {32, 32};
     const cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
+              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS
                ? QB200_OK : QB200_ERR_DRIVER;
 }
 
@@ -1336,13 +1246,13 @@ static void make_output_maps(CUtensorMap* map, PeerMaps<PUSH>* peers, EpiloguePa
     ep->tma_store = 1;
 }
 
-// A operand as int8 [rows, K] row-major; box = 128 bytes (one K stage, the swizzle span) x 256 rows.
-static int make_a8_map(CUtensorMap* map, const void* base, int rows, int K) {
+// A operand as int8 [rows, K] row-major; box = 128 bytes (one K stage, the swizzle span) x box_rows.
+static int make_a8_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows) {
     EncodeTiledFn fn = get_encode_fn();
     if (fn == nullptr) return QB200_ERR_DRIVER;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)K};
-    const cuuint32_t box[2] = {(cuuint32_t)U8_ROW, (cuuint32_t)wide::TM};
+    const cuuint32_t box[2] = {(cuuint32_t)U8_ROW, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1383,34 +1293,51 @@ static void wide_columns(EpilogueParams* ep, int M, int N, int sms, bool balance
     ep->col_rem = units % most;
 }
 
-static int launch_gemm_wide_a8(const EpilogueParams& ep_in, const void* a8, const void* b, int M, int K, int N, int sms,
-                               int dev, cudaStream_t stream) {
+// Tile columns of the pair kernel: multiples of 32, at most 256 wide, as many as fit the waves that 256-wide ones need.
+static void pair_columns(EpilogueParams* ep, int M, int N, int pairs) {
+    const int tiles_m = (M + pair2::TM - 1) / pair2::TM;
+    const int units = (N + 31) / 32;
+    int cols = (units + 7) / 8;
+    const long long waves = ((long long)tiles_m * cols + pairs - 1) / pairs;
+    long long most = waves * pairs / tiles_m;
+    if (most > units) most = units;
+    if (const char* e = getenv("QB200_GEMM_BALANCE"))
+        if (e[0] == '0') most = cols;
+    if (most > cols) cols = (int)most;
+    ep->col_count = cols;
+    ep->col_units = units / cols;
+    ep->col_rem = units % cols;
+}
+
+static int launch_gemm_pair(const EpilogueParams& ep_in, const void* a8, const void* b, int M, int K, int N, int sms, int dev,
+                            cudaStream_t stream) {
     EpilogueParams ep = ep_in;
     static bool attr_set[64] = {false};
-    auto kernel = gemm_i4_wide_kernel<true, false, true>;
+    auto kernel = gemm_i4_pair_kernel;
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_BYTES) != cudaSuccess)
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair2::SMEM_BYTES) != cudaSuccess)
             return QB200_ERR_CUDA;
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    CUtensorMap ma, mb;
-    int st = make_a8_map(&ma, a8, M, K);
+    const int pairs = sms / 2;
+    pair_columns(&ep, M, N, pairs);
+    const int b_box_rows = 16 * (ep.col_units + (ep.col_rem > 0 ? 1 : 0));  // half the widest tile
+    CUtensorMap ma, mb, md;
+    int st = make_a8_map(&ma, a8, M, K, pair2::CTA_ROWS);
     if (st != QB200_OK) return st;
-    st = make_packed_map(&mb, b, N, K, wide::TN);
+    st = make_packed_map(&mb, b, N, K, b_box_rows);
     if (st != QB200_OK) return st;
-    CUtensorMap md;
-    PeerMaps<false> peers;
-    make_output_maps<false>(&md, &peers, &ep, M, N);
-    CUtensorMap md16;
-    memset(&md16, 0, sizeof(md16));
-    ep.tma_store16 = 0;
-    if (ep.tma_store && encode_output_map16(&md16, ep.out, ep.ld, M, N) == QB200_OK) ep.tma_store16 = 1;
+    memset(&md, 0, sizeof(md));
+    ep.tma_store = aligned16(ep.out) && ep.ld % 8 == 0 && encode_output_map32(&md, ep.out, ep.ld, M, N) == QB200_OK;
     if (const char* e = getenv("QB200_GEMM_TMA_STORE"))
-        if (e[0] == '1') ep.tma_store16 = 0;  // 1: only the last tile of a CTA leaves through shared memory
-    wide_columns(&ep, M, N, sms, true);
-    const int tiles = ((M + wide::TM - 1) / wide::TM) * ep.col_count;
-    const int grid = tiles < sms ? tiles : sms;
-    if (launch_kernel(kernel, grid, wide::kThreads - 32, wide::SMEM_BYTES, stream, ma, mb, md, md16, peers, ep, M, N, K) != cudaSuccess) {
+        if (e[0] == '0') ep.tma_store = 0;
+    const int tiles_m = (M + pair2::TM - 1) / pair2::TM;
+    const long long tiles = (long long)tiles_m * ep.col_count;
+    int group = tiles_m <= 32 ? tiles_m : 16;
+    if (const char* e = getenv("QB200_GEMM_GROUP"))
+        if (atoi(e) > 0) group = atoi(e) < tiles_m ? atoi(e) : tiles_m;
+    const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
+    if (launch_kernel(kernel, grid, pair2::kThreads, pair2::SMEM_BYTES, stream, ma, mb, md, ep, M, N, K, b_box_rows, group) != cudaSuccess) {
         cudaGetLastError();
         return QB200_ERR_CUDA;
     }
@@ -1431,7 +1358,7 @@ static int launch_gemm_wide_impl(const EpilogueParams& ep_in, const void* a, con
     wide_columns(&ep, M, N, sms, FUSED, 8, 13, PUSH && ep.n_peer > 1 ? 4 : 1);
     const bool clip = ep.col_units < wide::TN / 16;
     static bool attr_set[2][64] = {{false}};
-    auto kernel = clip ? gemm_i4_wide_kernel<FUSED, PUSH, false, FUSED> : gemm_i4_wide_kernel<FUSED, PUSH, false, false>;
+    auto kernel = clip ? gemm_i4_wide_kernel<FUSED, PUSH, FUSED> : gemm_i4_wide_kernel<FUSED, PUSH, false>;
     if (dev < 0 || dev >= 64 || !attr_set[clip][dev]) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, wide::SMEM_BYTES) != cudaSuccess)
             return QB200_ERR_CUDA;
@@ -1453,7 +1380,7 @@ static int launch_gemm_wide_impl(const EpilogueParams& ep_in, const void* a, con
         memset(&md, 0, sizeof(md));
         memset(&peers, 0, sizeof(peers));
     }
-    if (launch_kernel(kernel, grid, threads, wide::SMEM_BYTES, stream, ma, mb, md, md, peers, ep, M, N, K) != cudaSuccess) {
+    if (launch_kernel(kernel, grid, threads, wide::SMEM_BYTES, stream, ma, mb, md, peers, ep, M, N, K) != cudaSuccess) {
         cudaGetLastError();
         return QB200_ERR_CUDA;
     }
@@ -1639,15 +1566,19 @@ static int dependent_launch_mask() {
     return e == nullptr ? -1 : atoi(e);
 }
 
+// Before a GEMM launch: inside a layer the kernel before it in the stream is the layer's quantiser.
+static void note_layer_launch(int M, int K) {
+    if (!tl_layer_mode) return;
+    const int mask = dependent_launch_mask();
+    const bool small = (long long)M * K < 3ll * 1024 * 1024;
+    tl_dependent_launch = mask >= 0 ? (mask & 1) != 0
+                                    : (qb_tl_quantiser_kernel == kQuantiserTc || (qb_tl_quantiser_kernel == kQuantiserMma && small));
+    qb_tl_quantiser_kernel = 0;  // consumed: a second GEMM of the layer follows a GEMM, not the quantiser
+}
+
 static int run_gemm(bool fused, const EpilogueParams& ep, const void* a, const void* b, int M, int K, int N,
                     cudaStream_t stream, int static_splits = -1) {
-    if (tl_layer_mode) {  // the kernel before this GEMM in the stream is the layer's quantiser
-        const int mask = dependent_launch_mask();
-        const bool small = (long long)M * K < 3ll * 1024 * 1024;
-        tl_dependent_launch = mask >= 0 ? (mask & 1) != 0
-                                        : (qb_tl_quantiser_kernel == kQuantiserTc || (qb_tl_quantiser_kernel == kQuantiserMma && small));
-        qb_tl_quantiser_kernel = 0;  // consumed: a second GEMM of the layer follows a GEMM, not the quantiser
-    }
+    note_layer_launch(M, K);
     const int st = run_gemm_impl(fused, ep, a, b, M, K, N, stream, static_splits);
     tl_dependent_launch = false;
     return st;
@@ -1719,12 +1650,8 @@ extern "C" int fused_matmul_dequantize_a8_int4t_bf16_cuda(void* mat_d, const voi
     int dev = 0;
     const int sms = sm_count_of_current_device(&dev);
     if (sms <= 0) return QB200_ERR_CUDA;
-    if (tl_layer_mode) {  // behind the layer's tcgen05 quantiser: dependent unless the environment says otherwise
-        const int mask = dependent_launch_mask();
-        tl_dependent_launch = mask < 0 || (mask & 1) != 0;
-        qb_tl_quantiser_kernel = 0;
-    }
-    const int st = launch_gemm_wide_a8(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
+    note_layer_launch(M, K);
+    const int st = launch_gemm_pair(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
     tl_dependent_launch = false;
     return st;
 }
@@ -1810,7 +1737,7 @@ extern "C" int w4a4_linear_hadamard_a8_bf16_cuda(void* mat_d, const void* x, con
                                                  const void* w_scale, void* a_int8, void* a_scale, void* a_int_row_sum,
                                                  int M, int K, int N, int block, cudaStream_t stream) {
     if (!a_int_row_sum) return QB200_ERR_INVALID_ARGUMENT;
-    quest_b200_begin_layer();  // the quantiser of this route is always the tcgen05 kernel: both launches dependent
+    quest_b200_begin_layer();
     int st = hadamard_quantize_a8_cuda_bf16(a_int8, a_scale, a_int_row_sum, x, K, M, block, stream);
     if (st == QB200_OK)
         st = fused_matmul_dequantize_a8_int4t_bf16_cuda(mat_d, a_int8, w_int_packed, a_int_row_sum, w_add, a_scale, w_scale,

@@ -1124,6 +1124,7 @@ extern "C" int hadamard_quantize_a8_cuda_bf16(void* a8_ptr, void* scale_ptr, voi
     p.M = batch_size;
     p.quantize = 1;
     p.had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)block))));
+    qb_tl_quantiser_kernel = kQuantiserTc;
     if (!hq_tc_eligible(p, block)) return QB200_ERR_UNSUPPORTED;  // only the tcgen05 kernel writes this format
     switch (block) {
         case 64: return launch_hq_tc<64>(p, stream);
