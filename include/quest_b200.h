@@ -191,6 +191,20 @@ int fused_matmul_dequantize_a8_int4t_bf16_cuda(void* mat_d, const void* mat_a8, 
 int quest_b200_prefers_a8(int M, int K, int N);
 
 /*
+ * 1 if a layer of this shape (w4a4_linear_hadamard_a8_bf16_cuda, which takes every K that is a multiple of its block and of
+ * 128) is faster on the int8 operand than on packed codes, else 0.
+ */
+int quest_b200_layer_operand(int M, int K, int N);
+
+/*
+ * The layer in one call with or without (block 0) the Hadamard transform, on packed codes ([M, K/2]) or, with int8_operand,
+ * on the int8 operand ([M, K]): what quest_b200.layer.linear_forward calls.
+ */
+int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add, const void* w_scale,
+                           void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M, int K, int N, int block,
+                           cudaStream_t stream);
+
+/*
  * Fused block-Hadamard + scale + int4 quantise + pack + row-sum of bf16 activations, one pass over
  * x.  Per row: xh = bf16(H_block . x) blockwise along K (Sylvester order, entries +-bf16(block^-0.5)),
  * scale = find_scale(xh), codes = quantize(xh, scale).  Replaces the three launches of the reference's

@@ -354,6 +354,11 @@ def prefers_a8(m: int, k: int, n: int) -> bool:
     return bool(_lib.load().quest_b200_prefers_a8(int(m), int(k), int(n)))
 
 
+def layer_operand(m: int, k: int, n: int) -> bool:
+    """Whether a whole layer of this shape (``linear_forward``, ``Linear4bit``) is faster on the int8 operand."""
+    return bool(_lib.load().quest_b200_layer_operand(int(m), int(k), int(n)))
+
+
 def hadamard_quantize_a8(
         x: torch.Tensor,
         block: int = 128,

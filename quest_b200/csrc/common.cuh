@@ -35,20 +35,36 @@ inline int launch_status() {
 __device__ __forceinline__ void wait_for_preceding_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// cluster > 0: in clusters of that many blocks along x (for kernels without a compile-time cluster size).
 template <typename Kernel, typename... Args>
-inline cudaError_t launch_kernel_dep(bool dependent, Kernel kernel, long long grid, int threads, size_t smem,
-                                     cudaStream_t stream, Args... args) {
+inline cudaError_t launch_kernel_cluster(bool dependent, int cluster, Kernel kernel, long long grid, int threads, size_t smem,
+                                         cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (dependent) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 0) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = dependent ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <typename Kernel, typename... Args>
+inline cudaError_t launch_kernel_dep(bool dependent, Kernel kernel, long long grid, int threads, size_t smem,
+                                     cudaStream_t stream, Args... args) {
+    return launch_kernel_cluster(dependent, 0, kernel, grid, threads, smem, stream, args...);
 }
 
 // Set (per host thread) by the one-call layer entry points around their quantiser call: the tcgen05 quantiser kernel
@@ -61,6 +77,10 @@ extern thread_local int qb_tl_quantiser_kernel;
 
 // Reads and clears the device status word of the row-kernel translation unit (see tcgen05.cuh).
 int hq_tc_fetch_and_clear_device_status(int* out);
+
+// The activation side of a layer on the int8-operand route: scale, quantise (behind the block transform; block 0: none) and
+// write the GEMM's operand.  Any K that is a multiple of 128.
+int quantise_layer_operand(void* a8, void* scale, void* row_sum, const void* x, int K, int M, int block, cudaStream_t stream);
 
 // Whether the tcgen05 quantiser can tile rows of K elements (block 128).
 bool hq_tc_shape_ok(int K);

@@ -1035,6 +1035,7 @@ gemm_i4_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 }
 
 #include "gemm_i4_pair.cuh"
+#include "gemm_i4_skinny.cuh"
 
 // ---------------------------------------------------------------------------------------------
 // Host side
@@ -1344,6 +1345,94 @@ static int launch_gemm_pair(const EpilogueParams& ep_in, const void* a8, const v
     return launch_status();
 }
 
+struct SkinnyPlan {
+    int rows, splits;
+    long long cycles;  // estimated
+};
+
+// Weight rows per CTA and K ranges of the skinny kernel, in cycles.  Measured (K = 4096, N = 11008 and 12288): a step of
+// 128 K takes 440 / 475 / 565 / 720 cycles of an SM at 16 / 32 / 64 / 128 tokens whatever the weight rows are (the issue
+// of four MMAs, then the tokens' way through shared memory), a launch about 8000 cycles, the exchange of a cluster 2500
+// and each wave of CTAs beyond the first about 3000.
+static SkinnyPlan pick_skinny(int tn, int K, int N, int sms) {
+    const int num_kb = K / BK;
+    const int per_sm = tn <= 32 ? 2 : 1;
+    const long long step = tn <= 16 ? 440 : (tn <= 32 ? 475 : (tn <= 64 ? 565 : 720));
+    SkinnyPlan best{0, 0, -1};
+    for (int s = 1; s <= skinny::kMaxSplit && s <= num_kb; ++s) {
+        // SMs that clusters of this size can use: the GPU's SMs come in groups of 16 to 20
+        const int usable = s <= 2 ? sms : sms - sms % 16;
+        for (int rows = skinny::W_ROWS; rows >= 8; rows -= 8) {
+            const long long ctas = (long long)((N + rows - 1) / rows) * s;
+            const long long waves = (ctas + (long long)usable * per_sm - 1) / ((long long)usable * per_sm);
+            const long long steps = (ctas + usable - 1) / usable * ((num_kb + s - 1) / s);  // of the busiest SM
+            const long long t = steps * step + 8000 + (waves - 1) * 3000 + (s > 1 ? 2500 : 0) + tn * 10;
+            if (best.cycles < 0 || t < best.cycles) best = SkinnyPlan{rows, s, t};
+        }
+    }
+    if (const char* e = getenv("QB200_SKINNY")) {  // tests, tuning: "rows,ranges"
+        int r = 0, s = 0;
+        if (sscanf(e, "%d,%d", &r, &s) == 2 && r >= 8 && r <= skinny::W_ROWS && r % 8 == 0 && s >= 1 && s <= skinny::kMaxSplit && s <= num_kb) best.rows = r, best.splits = s;
+    }
+    return best;
+}
+
+template <int TN>
+static int launch_gemm_skinny_tn(const EpilogueParams& ep, const void* a8, const void* b, int M, int K, int N, int sms, int dev,
+                                 cudaStream_t stream) {
+    using C = skinny::Cfg<TN>;
+    static bool attr_set[64] = {false};
+    auto kernel = gemm_i4_skinny_kernel<TN>;
+    if (dev < 0 || dev >= 64 || !attr_set[dev]) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess)
+            return QB200_ERR_CUDA;
+        if (dev >= 0 && dev < 64) attr_set[dev] = true;
+    }
+    const SkinnyPlan plan = pick_skinny(TN, K, N, sms);
+    CUtensorMap mw, mt;
+    int st = make_packed_map(&mw, b, N, K, plan.rows);
+    if (st != QB200_OK) return st;
+    st = make_a8_map(&mt, a8, M, K, TN);
+    if (st != QB200_OK) return st;
+    const long long grid = (long long)((N + plan.rows - 1) / plan.rows) * plan.splits;
+    if (launch_kernel_cluster(tl_dependent_launch, plan.splits > 1 ? plan.splits : 0, kernel, grid, skinny::kThreads, C::SMEM_BYTES,
+                              stream, mw, mt, ep, M, N, K, plan.rows, plan.splits) != cudaSuccess) {
+        cudaGetLastError();
+        return QB200_ERR_CUDA;
+    }
+    return launch_status();
+}
+
+static int skinny_tokens(int M) { return M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128)); }
+
+// Estimated cycles of the pair kernel: a 128-K step of a tile measured 260 + 1.3 cycles per column (at least 400), a
+// launch about 11000 cycles.
+static long long pair_cycles(int M, int K, int N, int sms) {
+    EpilogueParams cols{};
+    const int pairs = sms / 2;
+    pair_columns(&cols, M, N, pairs);
+    const long long width = 32ll * (cols.col_units + (cols.col_rem > 0 ? 1 : 0));
+    const long long tiles = (long long)((M + pair2::TM - 1) / pair2::TM) * cols.col_count;
+    long long step = 260 + width * 13 / 10;
+    if (step < 400) step = 400;
+    return (tiles + pairs - 1) / pairs * (K / BK) * step + 11000;
+}
+
+// The GEMM of the int8-operand route: the skinny kernel where its estimate is the shorter one (up to 128 rows), the pair
+// kernel elsewhere.  QB200_A8_KERNEL=pair|skinny forces one (tests, tuning).
+static int launch_gemm_a8(const EpilogueParams& ep, const void* a8, const void* b, int M, int K, int N, int sms, int dev,
+                          cudaStream_t stream) {
+    bool use_skinny = M <= 128 && pick_skinny(skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms);
+    if (const char* e = getenv("QB200_A8_KERNEL")) use_skinny = e[0] == 's' && M <= 128;
+    if (!use_skinny) return launch_gemm_pair(ep, a8, b, M, K, N, sms, dev, stream);
+    switch (skinny_tokens(M)) {
+        case 16: return launch_gemm_skinny_tn<16>(ep, a8, b, M, K, N, sms, dev, stream);
+        case 32: return launch_gemm_skinny_tn<32>(ep, a8, b, M, K, N, sms, dev, stream);
+        case 64: return launch_gemm_skinny_tn<64>(ep, a8, b, M, K, N, sms, dev, stream);
+        default: return launch_gemm_skinny_tn<128>(ep, a8, b, M, K, N, sms, dev, stream);
+    }
+}
+
 template <bool FUSED, bool PUSH>
 static int launch_gemm_wide_impl(const EpilogueParams& ep_in, const void* a, const void* b, int M, int K, int N, int sms,
                                  int dev, cudaStream_t stream) {
@@ -1651,11 +1740,12 @@ extern "C" int fused_matmul_dequantize_a8_int4t_bf16_cuda(void* mat_d, const voi
     const int sms = sm_count_of_current_device(&dev);
     if (sms <= 0) return QB200_ERR_CUDA;
     note_layer_launch(M, K);
-    const int st = launch_gemm_pair(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
+    const int st = launch_gemm_a8(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
     tl_dependent_launch = false;
     return st;
 }
 
+constexpr int kGemvRows = 4;  // of a layer; provisional
 constexpr bool kA8ByDefault = true;  // measured faster wherever the 256 x 256 kernel and the tcgen05 quantiser both apply (QB200_A8=0 switches it off)
 
 // 1 if, for this layer shape, the int8-operand route (hadamard_quantize_a8_cuda_bf16 + the GEMM above) is the faster one:
@@ -1674,6 +1764,18 @@ extern "C" int quest_b200_prefers_a8(int M, int K, int N) {
     // between the CTAs that share its rows.
     if ((long long)M * K > (48ll << 20)) return 0;
     return hq_tc_shape_ok(K) ? 1 : 0;
+}
+
+// 1 if the layer (quantiser and GEMM in one) takes the int8 operand: every K that is a multiple of 128, except for the
+// few rows where the dp4a kernel on packed codes is the faster one.
+extern "C" int quest_b200_layer_operand(int M, int K, int N) {
+    if (M <= 0 || K <= 0 || N <= 0 || K % 128 != 0 || K >= (1 << 17)) return 0;
+    if (getenv("QB200_GEMM_TILE") != nullptr || getenv("QB200_GEMM_SPLITS") != nullptr) return 0;
+    if (const char* e = getenv("QB200_A8")) return e[0] != '0';
+    int dev = 0;
+    const int sms = sm_count_of_current_device(&dev);
+    if (sms < 2) return 0;
+    return M > kGemvRows || !gemv_eligible(M, K, N, 0);
 }
 
 extern "C" int fused_matmul_dequantize_int4_int4t_bf16_noalloc_cuda(void* mat_d, const void* mat_a, const void* mat_b,
@@ -1731,17 +1833,34 @@ extern "C" int w4a4_linear_hadamard_bf16_cuda(void* mat_d, const void* x, const 
     return st;
 }
 
-extern "C" int hadamard_quantize_a8_cuda_bf16(void*, void*, void*, const void*, int, int, int, cudaStream_t);
-
 extern "C" int w4a4_linear_hadamard_a8_bf16_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add,
                                                  const void* w_scale, void* a_int8, void* a_scale, void* a_int_row_sum,
                                                  int M, int K, int N, int block, cudaStream_t stream) {
     if (!a_int_row_sum) return QB200_ERR_INVALID_ARGUMENT;
     quest_b200_begin_layer();
-    int st = hadamard_quantize_a8_cuda_bf16(a_int8, a_scale, a_int_row_sum, x, K, M, block, stream);
+    int st = quantise_layer_operand(a_int8, a_scale, a_int_row_sum, x, K, M, block, stream);
     if (st == QB200_OK)
         st = fused_matmul_dequantize_a8_int4t_bf16_cuda(mat_d, a_int8, w_int_packed, a_int_row_sum, w_add, a_scale, w_scale,
                                                         M, K, N, stream);
+    quest_b200_end_layer();
+    return st;
+}
+
+extern "C" int scale_quantize_int4_cuda_bf16(void*, void*, void*, const void*, int, int, int, int, cudaStream_t);
+
+extern "C" int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add, const void* w_scale,
+                                      void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M, int K, int N,
+                                      int block, cudaStream_t stream) {
+    if (block != 0)
+        return int8_operand ? w4a4_linear_hadamard_a8_bf16_cuda(mat_d, x, w_int_packed, w_add, w_scale, codes, a_scale, a_int_row_sum, M, K, N, block, stream)
+                            : w4a4_linear_hadamard_bf16_cuda(mat_d, x, w_int_packed, w_add, w_scale, codes, a_scale, a_int_row_sum, M, K, N, block, stream);
+    if (!a_int_row_sum) return QB200_ERR_INVALID_ARGUMENT;
+    quest_b200_begin_layer();
+    int st = int8_operand ? quantise_layer_operand(codes, a_scale, a_int_row_sum, x, K, M, 0, stream)
+                          : scale_quantize_int4_cuda_bf16(codes, a_scale, a_int_row_sum, x, K, M, 0, 0, stream);
+    if (st == QB200_OK)
+        st = int8_operand ? fused_matmul_dequantize_a8_int4t_bf16_cuda(mat_d, codes, w_int_packed, a_int_row_sum, w_add, a_scale, w_scale, M, K, N, stream)
+                          : fused_matmul_dequantize_int4_int4t_bf16_cuda(mat_d, codes, w_int_packed, a_int_row_sum, w_add, a_scale, w_scale, M, K, N, stream);
     quest_b200_end_layer();
     return st;
 }

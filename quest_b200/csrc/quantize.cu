@@ -26,7 +26,7 @@ struct RowParams {
     __nv_bfloat16* scale_out;      // optional [M] computed scale
     int8_t* q_dense;               // optional [M,K]
     uint8_t* q_packed;             // optional [M,K/2]
-    uint8_t* q_a8;                 // optional [M,K]: sixteen times the codes as int8, in the GEMM's operand order (tcgen05 kernel only)
+    uint8_t* q_a8;                 // optional [M,K]: sixteen times the codes as int8, in the GEMM's operand order (instead of q_packed)
     int32_t* row_sum;              // optional [M]
     int K;
     int M;
@@ -90,6 +90,12 @@ __device__ __forceinline__ int nibble_sum16(uint32_t w, int acc) {
     return acc;
 }
 
+// 32 packed codes as the GEMM's int8 operand: sixteen times the codes, the even positions of the group first (see q_a8).
+__device__ __forceinline__ void store_a8(uint8_t* dst, const uint4& w) {
+    *reinterpret_cast<uint4*>(dst) = make_uint4((w.x << 4) & 0xF0F0F0F0u, (w.y << 4) & 0xF0F0F0F0u, (w.z << 4) & 0xF0F0F0F0u, (w.w << 4) & 0xF0F0F0F0u);
+    *reinterpret_cast<uint4*>(dst + 16) = make_uint4(w.x & 0xF0F0F0F0u, w.y & 0xF0F0F0F0u, w.z & 0xF0F0F0F0u, w.w & 0xF0F0F0F0u);
+}
+
 template <int HB>
 __device__ __forceinline__ void hadamard32(float (&f)[32], int lane) {
     // Index bits 0..4 live in registers.
@@ -120,6 +126,7 @@ __device__ __forceinline__ void hadamard32(float (&f)[32], int lane) {
 // used outputs (dense int8 codes, transformed / dequantised bf16 values).
 template <int HB, int UNITS, bool EXTRAS>
 __global__ void __launch_bounds__(UNITS == 1 ? 256 : 512) row_kernel(const RowParams p) {
+    if (!EXTRAS) let_dependents_launch();  // the GEMM of a layer without the transform; it waits for this grid itself
     const int row = blockIdx.x;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -254,7 +261,9 @@ __global__ void __launch_bounds__(UNITS == 1 ? 256 : 512) row_kernel(const RowPa
                 }
             }
         }
-        if (p.q_packed != nullptr) {
+        if (!EXTRAS && p.q_a8 != nullptr) {  // K is a multiple of 128 here
+            if (e0 < K) store_a8(p.q_a8 + (size_t)row * K + e0, make_uint4(pk[0], pk[1], pk[2], pk[3]));
+        } else if (p.q_packed != nullptr) {
             uint8_t* dst = p.q_packed + (size_t)row * (K >> 1) + (e0 >> 1);
             if (vec_store) {
                 if (e0 < K) *reinterpret_cast<uint4*>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
@@ -647,7 +656,9 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
             rs16 = nibble_sum16(w.z, rs16);
             rs16 = nibble_sum16(w.w, rs16);
             const int e0 = unit * kUnit + lane * 32;
-            if (row < M) {
+            if (row < M && p.q_a8 != nullptr) {  // K is a multiple of 128 here
+                if (e0 < K) store_a8(p.q_a8 + (size_t)row * K + e0, w);
+            } else if (row < M) {
                 uint8_t* dst = p.q_packed + (size_t)row * (K >> 1) + (e0 >> 1);
                 if (vec_store) {
                     if (e0 < K) *reinterpret_cast<uint4*>(dst) = w;
@@ -853,6 +864,7 @@ static bool vector_path_ok(const RowParams& p) {
     if (p.x_out != nullptr && !aligned16(p.x_out)) return false;
     if (p.q_dense != nullptr && (reinterpret_cast<uintptr_t>(p.q_dense) & 7u)) return false;
     if (p.q_packed != nullptr && !aligned16(p.q_packed)) return false;
+    if (p.q_a8 != nullptr && (!aligned16(p.q_a8) || p.K % 128 != 0)) return false;
     return true;
 }
 
@@ -1002,6 +1014,8 @@ extern "C" int quantize_int4_cuda_bf16(void* x_ptr, const void* scale_ptr, void*
     return run_rows(p, 0, extras, stream);
 }
 
+constexpr long long kTcFromInLayer = 3ll * 1024 * 1024;  // see the crossover below
+
 extern "C" int hadamard_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* scale_ptr, void* x_int_row_sum_ptr,
                                                 const void* x_ptr, int group_size, int batch_size, int block,
                                                 cudaStream_t stream) {
@@ -1028,7 +1042,7 @@ extern "C" int hadamard_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* sc
     // kernel and the GEMM behind it are launched with programmatic dependencies, which gains more than that
     // microsecond (M = 1024, K = N = 4096: 27.2 against 28.2 us per layer), while a GEMM launched that way behind
     // the CUDA-core kernel measured slower from 4 M elements on (29.5 us).
-    const long long tc_from = qb_tl_dependent_quantiser ? 3ll * 1024 * 1024 : 12ll * 1024 * 1024;
+    const long long tc_from = qb_tl_dependent_quantiser ? kTcFromInLayer : 12ll * 1024 * 1024;
     const bool want_tc = force != nullptr ? (force[0] == 't') : ((long long)p.M * p.K >= tc_from);
     if (want_tc && hq_tc_eligible(p, block)) {
         qb_tl_quantiser_kernel = kQuantiserTc;
@@ -1124,14 +1138,45 @@ extern "C" int hadamard_quantize_a8_cuda_bf16(void* a8_ptr, void* scale_ptr, voi
     p.M = batch_size;
     p.quantize = 1;
     p.had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)block))));
+    if (!hq_tc_eligible(p, block)) return QB200_ERR_UNSUPPORTED;
     qb_tl_quantiser_kernel = kQuantiserTc;
-    if (!hq_tc_eligible(p, block)) return QB200_ERR_UNSUPPORTED;  // only the tcgen05 kernel writes this format
     switch (block) {
         case 64: return launch_hq_tc<64>(p, stream);
         case 128: return launch_hq_tc<128>(p, stream);
         default: return launch_hq_tc<256>(p, stream);
     }
 }
+
+namespace qb {
+int quantise_layer_operand(void* a8, void* scale, void* row_sum, const void* x, int K, int M, int block, cudaStream_t stream) {
+    if (K < 0 || M < 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (block != 0 && block != 64 && block != 128 && block != 256) return QB200_ERR_UNSUPPORTED;
+    if (M == 0) return QB200_OK;
+    if (a8 == nullptr || scale == nullptr || x == nullptr || K == 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (block != 0 && K % block != 0) return QB200_ERR_INVALID_ARGUMENT;
+    RowParams p{};
+    p.x = static_cast<const __nv_bfloat16*>(x);
+    p.scale_out = static_cast<__nv_bfloat16*>(scale);
+    p.q_a8 = static_cast<uint8_t*>(a8);
+    p.row_sum = static_cast<int32_t*>(row_sum);
+    p.K = K;
+    p.M = M;
+    p.quantize = 1;
+    if (!vector_path_ok(p)) return QB200_ERR_UNSUPPORTED;
+    if (block == 0) {
+        qb_tl_quantiser_kernel = kQuantiserMma;
+        return run_rows(p, 0, false, stream);
+    }
+    p.had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)block))));
+    const bool tc = hq_tc_eligible(p, block) && (long long)M * K >= kTcFromInLayer;
+    qb_tl_quantiser_kernel = tc ? kQuantiserTc : kQuantiserMma;
+    switch (block) {
+        case 64: return tc ? launch_hq_tc<64>(p, stream) : launch_hq_mma<64>(p, stream);
+        case 128: return tc ? launch_hq_tc<128>(p, stream) : launch_hq_mma<128>(p, stream);
+        default: return tc ? launch_hq_tc<256>(p, stream) : launch_hq_mma<256>(p, stream);
+    }
+}
+}  // namespace qb
 
 extern "C" int hadamard_transform_cuda_bf16(void* out_ptr, const void* x_ptr, int group_size, int batch_size,
                                             int block, int weight_side, cudaStream_t stream) {

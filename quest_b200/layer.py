@@ -13,6 +13,7 @@ import torch
 from torch import nn
 
 import quest_b200 as quest
+from . import _lib
 from .workspace import default_cache
 
 HADAMARD_BLOCK = 128  # the reference hard-codes block 128 (utils.py:17, 39, 90)
@@ -87,6 +88,60 @@ def _one_call_ok(*tensors: torch.Tensor) -> bool:
     return all(t.is_contiguous() for t in tensors)
 
 
+_BLOCKS = (64, 128, 256)
+
+
+def _layer_call(x, w, w_scale, w_add, out, ws, block):
+    """The whole layer as one library call, or None where its buffers are not what that call takes (linear_forward then goes
+    through the single ops, which check and report).  ``block`` 0: no transform.  ``ws``: None, or (codes, scale, row sums)
+    where codes [M, K] selects the int8 operand and [M, K/2] packed int4; None takes one allocation for all three."""
+    if x.dim() != 2 or w.dim() != 2 or not x.is_cuda:
+        return None
+    (m, k), n, dev = x.shape, w.size(0), x.get_device()
+    if (m == 0 or n == 0 or k == 0 or k > 65536 or w.size(1) * 2 != k or (k % block if block else k % 32)
+            or x.dtype is not torch.bfloat16 or w.dtype is not torch.uint8 or w_scale.dtype is not torch.bfloat16
+            or w_add.dtype is not torch.int32 or w_scale.numel() != n or w_add.numel() != n
+            or w.get_device() != dev or w_scale.get_device() != dev or w_add.get_device() != dev
+            or not (x.is_contiguous() and w.is_contiguous() and w_scale.is_contiguous() and w_add.is_contiguous())):
+        return None
+    xp, wp = x.data_ptr(), w.data_ptr()
+    if xp % 16 or wp % 16:
+        return None
+    if out is None:
+        out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+    elif out.shape != (m, n) or out.dtype is not torch.bfloat16 or out.get_device() != dev or not out.is_contiguous():
+        return None
+    lib = _lib.load()
+    if ws is None:
+        int8 = lib.quest_b200_layer_operand(m, k, n)
+        code_bytes = -(-(m * k if int8 else m * (k // 2)) // 256) * 256
+        buf = torch.empty(code_bytes + 6 * m, dtype=torch.uint8, device=x.device)
+        codes = buf.data_ptr()
+        sums = codes + code_bytes
+        scale = sums + 4 * m
+    else:
+        a, a_scale, a_sums = ws
+        if (a.shape not in ((m, k), (m, k // 2)) or a.dtype is not torch.uint8 or a_scale.dtype is not torch.bfloat16
+                or a_sums.dtype is not torch.int32 or a_scale.numel() != m or a_sums.numel() != m
+                or a.get_device() != dev or a_scale.get_device() != dev or a_sums.get_device() != dev
+                or not (a.is_contiguous() and a_scale.is_contiguous() and a_sums.is_contiguous()) or a.data_ptr() % 16):
+            return None
+        int8 = int(a.size(1) == k)
+        codes, scale, sums = a.data_ptr(), a_scale.data_ptr(), a_sums.data_ptr()
+    if int8 and k % 128:
+        return None
+    args = (out.data_ptr(), xp, wp, w_add.data_ptr(), w_scale.data_ptr(), codes, int8, scale, sums, m, k, n, block,
+            torch._C._cuda_getCurrentRawStream(dev))
+    if torch._C._cuda_getDevice() == dev:
+        status = lib.w4a4_linear_layer_cuda(*args)
+    else:
+        with torch.cuda.device(dev):
+            status = lib.w4a4_linear_layer_cuda(*args)
+    if status:
+        _lib.check(status, "w4a4_linear_layer_cuda")
+    return out
+
+
 def linear_forward(
         activation: torch.Tensor,
         w_int_packed: torch.Tensor,
@@ -109,14 +164,26 @@ def linear_forward(
     fused kernel is used whether or not ``_c`` is given; ``debug_mode=True`` (not in the reference's signature)
     takes the unfused int32 GEMM + add_mul_vv route with ``_c`` as its int32 workspace.
 
-    With ``use_hadamard`` and a shape for which the library prefers it, the quantiser writes the GEMM's int8 operand
-    directly (``_a_int8`` [M, K] uint8 is its workspace) instead of packed int4: same codes, same result, no unpack
-    of A inside the GEMM.  A caller that passes ``_a_int_packed`` but no ``_a_int8`` keeps the packed route.
+    Where the library finds it faster the quantiser writes the GEMM's int8 operand directly (``_a_int8`` [M, K] uint8 is its
+    workspace) instead of packed int4: same codes, same result, no unpack of A inside the GEMM.  A caller that passes
+    ``_a_int_packed`` but no ``_a_int8`` keeps the packed route.
 
-    With ``use_hadamard`` (and dense buffers) the layer is ONE library call: the quantiser, then the GEMM kernel launched
-    with a programmatic dependency on it, so that the GEMM's set-up and first weight copies overlap the quantiser's end."""
+    With dense buffers the layer is ONE library call (``_layer_call``): the quantiser (with or without the transform, each
+    row read once), then the GEMM kernel, where it pays launched with a programmatic dependency on the quantiser so that
+    its set-up and first weight copies overlap the quantiser's end."""
     if w_meta_e is not None:
         raise NotImplementedError("quest_b200 implements the dense W4A4 path only")
+    if not debug_mode and (not use_hadamard or block in _BLOCKS):
+        codes = _a_int_packed if _a_int8 is None else _a_int8
+        if _a_int8 is not None and _a_int_packed is not None and not quest.prefers_a8(*activation.shape, w_int_packed.size(0)):
+            codes = _a_int_packed
+        ws = None
+        if codes is not None and _a_scale is not None and _a_int_row_sum is not None:
+            ws = (codes, _a_scale, _a_int_row_sum)
+        if ws is not None or (codes is None and _a_scale is None and _a_int_row_sum is None):
+            y = _layer_call(activation, w_int_packed, w_scale, w_add, out, ws, block if use_hadamard else 0)
+            if y is not None:
+                return y
     M, K, N = activation.size(0), activation.size(1), w_int_packed.size(0)
     dtype, device = activation.dtype, activation.device
     if out is None:
@@ -200,7 +267,7 @@ class Linear4bit(nn.Module):
             a = x.contiguous().flatten(end_dim=-2)
             # activation-side workspaces come from the shared per-stream cache: nothing but the output is allocated
             m, k = a.shape
-            a8 = self.use_hadamard and k % HADAMARD_BLOCK == 0 and quest.prefers_a8(m, k, self.out_features)
+            a8 = quest.layer_operand(m, k, self.out_features)
             ws = self.workspaces.get(m, k, a.device, a.dtype, int8_operand=a8)
             y = linear_forward(activation=a, w_int_packed=self.w_int_packed, w_scale=self.w_scale, w_add=self.w_add,
                                w_meta_e=self.w_meta_e, out=None, use_hadamard=self.use_hadamard, **ws)
