@@ -297,6 +297,23 @@ int hadamard_transform_cuda_bf16(void* out_ptr, const void* x_ptr, int group_siz
 int scale_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* scale_ptr, void* x_int_row_sum_ptr, const void* x_ptr,
                                   int group_size, int batch_size, int weight_block, int row_sum_add, cudaStream_t stream);
 
+/*
+ * Rotary embedding in place: x[r, 2j], x[r, 2j+1] of the first `cols` columns (whole heads of head_dim) of every row are
+ * rotated by table[r % seq, j % (head_dim/2)] = (cos, sin), fp32 or bf16 (src/models/llama.py:43-62, same roundings).
+ * head_dim and ld multiples of 8, x and table 16-byte aligned (QB200_ERR_UNSUPPORTED otherwise).
+ */
+int rope_inplace_cuda_bf16(void* x, const void* table, int table_is_bf16, int rows, int seq, int cols, int head_dim,
+                           long long ld, cudaStream_t stream);
+
+/*
+ * The producer-fused quantisers in one entry.  producer 1: RMSNorm(x) * norm_weight; 2: SiLU(x) * x2; 3: sum = bf16(x + x2),
+ * written to sum_ptr (which may be x2), then RMSNorm(sum) * norm_weight.  int8_operand != 0: codes_ptr is [M, K] bytes
+ * and receives the GEMM's int8 operand (see hadamard_quantize_a8_cuda_bf16) instead of [M, K/2] packed codes.
+ */
+int producer_hadamard_quantize_cuda_bf16(void* codes_ptr, int int8_operand, void* scale_ptr, void* x_int_row_sum_ptr, int producer,
+                                         const void* x_ptr, const void* x2_ptr, void* sum_ptr, const void* norm_weight_ptr,
+                                         float eps, int group_size, int batch_size, int block, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -284,6 +284,53 @@ def silu_mul_hadamard_quantize_int4(
     return x_int_packed, scale, x_int_row_sum
 
 
+PRODUCE_RMSNORM, PRODUCE_SILU_MUL, _PRODUCE_ADD_RMSNORM = 1, 2, 3
+
+
+def producer_hadamard_quantize(
+        producer: int,
+        x: torch.Tensor,
+        codes: torch.Tensor,
+        scale: torch.Tensor,
+        x_int_row_sum: torch.Tensor,
+        x2: torch.Tensor = None,
+        norm_weight: torch.Tensor = None,
+        eps: float = 0.0,
+        block: int = 128,
+        _sum: torch.Tensor = None,
+) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """The producer-fused quantisers on caller-owned outputs: ``codes`` [M, K/2] receives packed int4, ``codes`` [M, K] the
+    GEMM's int8 operand.  PRODUCE_RMSNORM: of RMSNorm(x) * norm_weight; PRODUCE_SILU_MUL: of silu(x) * x2."""
+    assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.is_contiguous()
+    assert x2 is None or (x2.shape == x.shape and x2.dtype == torch.bfloat16 and x2.is_contiguous())
+    assert norm_weight is None or (norm_weight.dtype == torch.bfloat16 and norm_weight.is_contiguous() and norm_weight.numel() == x.size(1))
+    m, k = x.shape
+    assert codes.dtype == torch.uint8 and scale.dtype == torch.bfloat16 and x_int_row_sum.dtype == torch.int32
+    assert codes.is_contiguous() and scale.is_contiguous() and x_int_row_sum.is_contiguous()
+    assert codes.shape in ((m, k // 2), (m, k)) and scale.numel() == m and x_int_row_sum.numel() == m
+    dev = _lib.require_cuda(x, x2, norm_weight, codes, scale, x_int_row_sum)
+    _call("producer_hadamard_quantize_cuda_bf16", dev, _lib.ptr(codes), int(codes.size(1) == k), _lib.ptr(scale),
+          _lib.ptr(x_int_row_sum), int(producer), _lib.ptr(x), _lib.ptr(x2), _lib.ptr(_sum), _lib.ptr(norm_weight), float(eps),
+          k, m, int(block), _lib.stream_of(x))
+    return codes, scale, x_int_row_sum
+
+
+def add_rmsnorm_hadamard_quantize(
+        x: torch.Tensor,
+        y: torch.Tensor,
+        norm_weight: torch.Tensor,
+        eps: float,
+        codes: torch.Tensor,
+        scale: torch.Tensor,
+        x_int_row_sum: torch.Tensor,
+        block: int = 128,
+) -> tuple[torch.Tensor, tuple[torch.Tensor, torch.Tensor, torch.Tensor]]:
+    """(x + y, quantised RMSNorm(x + y) * norm_weight) in one pass; ``codes`` as in ``producer_hadamard_quantize``."""
+    total = torch.empty_like(x)
+    return total, producer_hadamard_quantize(_PRODUCE_ADD_RMSNORM, x, codes, scale, x_int_row_sum, x2=y, norm_weight=norm_weight,
+                                             eps=eps, block=block, _sum=total)
+
+
 def w4a4_linear_hadamard(
         x: torch.Tensor,
         w_int_packed: torch.Tensor,
@@ -431,6 +478,17 @@ def one_pass_ok(x: torch.Tensor, weight_block: int = 0) -> bool:
     """Whether ``scale_quantize_int4`` takes x: bf16 rows of whole 16-byte pieces that one block can hold."""
     return (x.dim() == 2 and x.dtype == torch.bfloat16 and x.is_contiguous() and 0 < x.size(1) <= 65536 and x.size(1) % 8 == 0
             and (weight_block == 0 or weight_block in (64, 128, 256) and x.size(1) % weight_block == 0) and x.data_ptr() % 16 == 0)
+
+
+def rope_inplace(x: torch.Tensor, table: torch.Tensor, seq: int, cols: int) -> torch.Tensor:
+    """Rotates the heads in the first ``cols`` columns of x [rows, ld] bf16 in place; row r is position r % seq of ``table``
+    (length, head_dim/2, 2), fp32 or bf16.  The same bits as the eager form of src/models/llama.py:43-62."""
+    assert x.dim() == 2 and x.dtype == torch.bfloat16 and x.is_contiguous() and table.is_contiguous()
+    assert table.dtype in (torch.bfloat16, torch.float32) and table.dim() == 3 and table.size(2) == 2 and seq <= table.size(0)
+    dev = _lib.require_cuda(x, table)
+    _call("rope_inplace_cuda_bf16", dev, _lib.ptr(x), _lib.ptr(table), int(table.dtype == torch.bfloat16), x.size(0), int(seq),
+          int(cols), 2 * table.size(1), x.size(1), _lib.stream_of(x))
+    return x
 
 
 def hadamard_transform(x: torch.Tensor, block: int = 128, weight_side: bool = False, out: torch.Tensor = None) -> torch.Tensor:

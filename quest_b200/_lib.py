@@ -39,6 +39,8 @@ SIGNATURES = {
     "quest_b200_end_layer": [],
     "hadamard_transform_cuda_bf16": [_P, _P, _I, _I, _I, _I, _P],
     "scale_quantize_int4_cuda_bf16": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "rope_inplace_cuda_bf16": [_P, _P, _I, _I, _I, _I, _I, _LL, _P],
+    "producer_hadamard_quantize_cuda_bf16": [_P, _I, _P, _P, _I, _P, _P, _P, _P, ctypes.c_float, _I, _I, _I, _P],
     "quest_b200_test_bounded_wait_cuda": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _LL, _P],
     "quest_b200_device_status": [ctypes.POINTER(ctypes.c_int)],
     "quest_b200_version": [],

@@ -358,11 +358,13 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm(
 //   0  the input itself.
 //   1  RMSNorm of the input:  y = bf16( bf16(x * rsqrt(mean(x^2) + eps)) * w )   (src/models/llama.py:64-76: the
 //      normalised value is cast back to the activation type before the weight multiplies it).
+//   3  the residual add in front of the norm as well: x + x2 is rounded to bf16, written to x_out (which may be x2) and
+//      normalised as in 1.
 //   2  SwiGLU gate:           y = bf16( bf16(silu(x)) * x2 ),  silu(x) = x / (1 + exp(-x)) in fp32
 //      (src/models/llama.py:118, torch's silu for bf16 inputs).
 // The producer rewrites the row in shared memory, in place, between the copy and the tensor-core stage; everything
 // after it is unchanged.  It saves the producer's own kernel(s), one write and one read of [M, K] bf16.
-constexpr int kProNone = 0, kProRmsNorm = 1, kProSiluMul = 2;
+constexpr int kProNone = 0, kProRmsNorm = 1, kProSiluMul = 2, kProAddRmsNorm = 3;
 
 template <int HB, int UNITS, int PRO = kProNone>
 __global__ void __launch_bounds__(256, UNITS == 1 ? 4 : (UNITS == 2 ? 3 : 2))
@@ -451,8 +453,9 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
 
         if (PRO != kProNone) {
             // Each lane owns the 16-byte chunks it copied itself (chunk c = 32 j + lane of every unit).
+            constexpr bool kNorm = PRO == kProRmsNorm || PRO == kProAddRmsNorm;
             float rinv = 0.f;
-            if (PRO == kProRmsNorm) {
+            if (kNorm) {
                 float nsq = 0.f;
 #pragma unroll
                 for (int u = 0; u < UNITS; ++u) {
@@ -460,8 +463,20 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int c = j * 32 + lane;
-                        const uint4 q = lds128(in_base + (c >> 4) * kBlkPitch + (c & 15) * 16);  // zero beyond K
-                        const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+                        const uint32_t addr = in_base + (c >> 4) * kBlkPitch + (c & 15) * 16;
+                        const uint4 q = lds128(addr);  // zero beyond K
+                        uint32_t w4[4] = {q.x, q.y, q.z, q.w};
+                        const int e = (u * W + wig) * kUnit + c * 8;
+                        if (PRO == kProAddRmsNorm && e < K && row < M) {
+                            const uint4 o = *reinterpret_cast<const uint4*>(p.x2 + (size_t)row * K + e);
+                            const uint32_t o4[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                w4[i] = pack_bf16x2(bf16lo_to_f32(w4[i]) + bf16lo_to_f32(o4[i]), bf16hi_to_f32(w4[i]) + bf16hi_to_f32(o4[i]));
+                            const uint4 sum = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                            *reinterpret_cast<uint4*>(p.x_out + (size_t)row * K + e) = sum;
+                            sts128(addr, sum);
+                        }
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             const float a = bf16lo_to_f32(w4[i]), b = bf16hi_to_f32(w4[i]);
@@ -493,14 +508,14 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
                     if (e >= K || row_p >= M) continue;
                     const uint32_t addr = in_base + (c >> 4) * kBlkPitch + (c & 15) * 16;
                     const uint4 q = lds128(addr);
-                    const uint4 o = PRO == kProRmsNorm ? __ldg(reinterpret_cast<const uint4*>(p.norm_w + e))
+                    const uint4 o = kNorm ? __ldg(reinterpret_cast<const uint4*>(p.norm_w + e))
                                                        : ld_stream16(p.x2 + (size_t)row_p * K + e);
                     const uint32_t w4[4] = {q.x, q.y, q.z, q.w}, o4[4] = {o.x, o.y, o.z, o.w};
                     uint32_t y4[4];
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         float a = bf16lo_to_f32(w4[i]), b = bf16hi_to_f32(w4[i]);
-                        if (PRO == kProRmsNorm) {
+                        if (kNorm) {
                             a *= rinv;
                             b *= rinv;
                         } else {
@@ -960,6 +975,42 @@ __global__ void copy_block_kernel(const uint8_t* __restrict__ src, const CopyDst
     }
 }
 
+// -------------------------------------------------------------------------------------------------
+// Rotary embedding of q and k where the fused projection has left them (columns [0, cols) of each qkv row), in place.
+// HBM-bound: one read and one write of q and k, 4 bytes per element, against a dozen passes in fp32 of the eager form.
+// The same roundings as the eager form: each product, the difference / sum and the conversion to bf16 are rounded once.
+// One thread owns four consecutive pairs (16 bytes); the table row of a position (head_dim * 8 bytes at most) stays in L1.
+// -------------------------------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(256) rope_inplace_kernel(__nv_bfloat16* __restrict__ x, const T* __restrict__ table,
+                                                           const long long chunks, const int row_chunks, const int seq,
+                                                           const long long ld, const int head_dim) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < chunks; i += (long long)gridDim.x * blockDim.x) {
+        const long long row = i / row_chunks;
+        const int col = (int)(i - row * row_chunks) * 8;
+        const T* t = table + (size_t)(row % seq) * head_dim + col % head_dim;  // (cos, sin) of the chunk's four pairs
+        float cs[8];
+        if (sizeof(T) == 4) {
+            const float4 a = __ldg(reinterpret_cast<const float4*>(t)), b = __ldg(reinterpret_cast<const float4*>(t) + 1);
+            cs[0] = a.x; cs[1] = a.y; cs[2] = a.z; cs[3] = a.w; cs[4] = b.x; cs[5] = b.y; cs[6] = b.z; cs[7] = b.w;
+        } else {
+            const uint4 a = __ldg(reinterpret_cast<const uint4*>(t));
+            const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) cs[2 * j] = bf16lo_to_f32(w[j]), cs[2 * j + 1] = bf16hi_to_f32(w[j]);
+        }
+        uint4* p = reinterpret_cast<uint4*>(x + row * ld + col);
+        const uint4 v = *p;
+        uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float x0 = bf16lo_to_f32(w[j]), x1 = bf16hi_to_f32(w[j]), c = cs[2 * j], s = cs[2 * j + 1];
+            w[j] = pack_bf16x2(__fsub_rn(__fmul_rn(x0, c), __fmul_rn(x1, s)), __fadd_rn(__fmul_rn(x0, s), __fmul_rn(x1, c)));
+        }
+        *p = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
 }  // namespace qb
 
 // -------------------------------------------------------------------------------------------------
@@ -1067,6 +1118,14 @@ static int run_producer_hq(RowParams& p, int block, int pro, cudaStream_t stream
     p.quantize = 1;
     p.had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)block))));
     if (!vector_path_ok(p)) return QB200_ERR_UNSUPPORTED;
+    if (pro == kProAddRmsNorm) {
+        if (!aligned16(p.norm_w) || !aligned16(p.x2)) return QB200_ERR_UNSUPPORTED;
+        switch (block) {
+            case 64: return launch_hq_mma<64, kProAddRmsNorm>(p, stream);
+            case 128: return launch_hq_mma<128, kProAddRmsNorm>(p, stream);
+            default: return launch_hq_mma<256, kProAddRmsNorm>(p, stream);
+        }
+    }
     if (pro == kProRmsNorm) {
         if (!aligned16(p.norm_w)) return QB200_ERR_UNSUPPORTED;
         switch (block) {
@@ -1101,6 +1160,33 @@ extern "C" int rmsnorm_hadamard_quantize_int4_cuda_bf16(void* x_int_packed_ptr, 
     p.K = group_size;
     p.M = batch_size;
     return run_producer_hq(p, block, kProRmsNorm, stream);
+}
+
+extern "C" int producer_hadamard_quantize_cuda_bf16(void* codes_ptr, int int8_operand, void* scale_ptr, void* x_int_row_sum_ptr,
+                                                    int producer, const void* x_ptr, const void* x2_ptr, void* sum_ptr,
+                                                    const void* norm_weight_ptr, float eps, int group_size, int batch_size,
+                                                    int block, cudaStream_t stream) {
+    if (group_size < 0 || batch_size < 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (block != 64 && block != 128 && block != 256) return QB200_ERR_UNSUPPORTED;
+    if (producer != kProRmsNorm && producer != kProSiluMul && producer != kProAddRmsNorm) return QB200_ERR_UNSUPPORTED;
+    if (batch_size == 0) return QB200_OK;
+    if (!codes_ptr || !scale_ptr || !x_ptr || group_size == 0 || group_size % block != 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (producer != kProSiluMul && !norm_weight_ptr) return QB200_ERR_INVALID_ARGUMENT;
+    if (producer != kProRmsNorm && !x2_ptr) return QB200_ERR_INVALID_ARGUMENT;
+    if (producer == kProAddRmsNorm && !sum_ptr) return QB200_ERR_INVALID_ARGUMENT;
+    RowParams p{};
+    p.x = static_cast<const __nv_bfloat16*>(x_ptr);
+    p.x2 = static_cast<const __nv_bfloat16*>(x2_ptr);
+    p.x_out = producer == kProAddRmsNorm ? static_cast<__nv_bfloat16*>(sum_ptr) : nullptr;
+    p.norm_w = static_cast<const __nv_bfloat16*>(norm_weight_ptr);
+    p.norm_eps = eps;
+    p.scale_out = static_cast<__nv_bfloat16*>(scale_ptr);
+    if (int8_operand) p.q_a8 = static_cast<uint8_t*>(codes_ptr);
+    else p.q_packed = static_cast<uint8_t*>(codes_ptr);
+    p.row_sum = static_cast<int32_t*>(x_int_row_sum_ptr);
+    p.K = group_size;
+    p.M = batch_size;
+    return run_producer_hq(p, block, producer, stream);
 }
 
 extern "C" int silu_mul_hadamard_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* scale_ptr, void* x_int_row_sum_ptr,
@@ -1241,6 +1327,23 @@ extern "C" int add_mul_vv_cuda_bf16(void* mat_d, const void* vec_a_add, const vo
         add_mul_vv_vec8_kernel<<<(unsigned)blocks, 256, 0, stream>>>(d, aa, am, ba, bm, c, size_a, size_b);
     else
         add_mul_vv_scalar_kernel<<<(unsigned)blocks, 256, 0, stream>>>(d, aa, am, ba, bm, c, size_a, size_b);
+    return launch_status();
+}
+
+extern "C" int rope_inplace_cuda_bf16(void* x, const void* table, int table_is_bf16, int rows, int seq, int cols, int head_dim,
+                                      long long ld, cudaStream_t stream) {
+    if (rows < 0 || cols < 0 || seq <= 0 || head_dim <= 0 || ld < cols) return QB200_ERR_INVALID_ARGUMENT;
+    if (rows == 0 || cols == 0) return QB200_OK;
+    if (!x || !table) return QB200_ERR_INVALID_ARGUMENT;
+    if (head_dim % 8 != 0 || cols % head_dim != 0 || ld % 8 != 0 || !aligned16(x) || !aligned16(table)) return QB200_ERR_UNSUPPORTED;
+    const long long chunks = (long long)rows * (cols / 8);
+    long long blocks = (chunks + 255) / 256;
+    if (blocks > 148 * 64) blocks = 148 * 64;
+    auto* p = static_cast<__nv_bfloat16*>(x);
+    if (table_is_bf16)
+        rope_inplace_kernel<__nv_bfloat16><<<(unsigned)blocks, 256, 0, stream>>>(p, static_cast<const __nv_bfloat16*>(table), chunks, cols / 8, seq, ld, head_dim);
+    else
+        rope_inplace_kernel<float><<<(unsigned)blocks, 256, 0, stream>>>(p, static_cast<const float*>(table), chunks, cols / 8, seq, ld, head_dim);
     return launch_status();
 }
 

@@ -255,7 +255,14 @@ class Linear4bit(nn.Module):
                           out: torch.Tensor = None) -> torch.Tensor:
         """The layer on activations that are already quantised ([M, K/2] packed codes, [M, 1] scales and row sums, as
         written by ``hadamard_quantize_int4`` or one of its producer-fused variants): only the fused GEMM runs.  Several
-        layers that read the same activations (w1 and w2 of a SwiGLU block) can share one quantisation this way."""
+        layers that read the same activations (w1 and w2 of a SwiGLU block) can share one quantisation this way.
+        ``a_int_packed`` [M, K] instead of [M, K/2] is the int8 operand (``producer_hadamard_quantize``)."""
+        if a_int_packed.size(1) == self.in_features:
+            y = quest.fused_matmul_dequantize_a8(mat_a8=a_int_packed, mat_b=self.w_int_packed, vec_a_add=a_int_row_sum,
+                                                 vec_b_add=self.w_add, vec_a_mul=a_scale, vec_b_mul=self.w_scale, out=out)
+            if self.bias is not None:
+                y += self.bias
+            return y
         y = quest.fused_matmul_dequantize_int4_int4t_bf16(mat_a=a_int_packed, mat_b=self.w_int_packed, vec_a_add=a_int_row_sum,
                                                           vec_b_add=self.w_add, vec_a_mul=a_scale, vec_b_mul=self.w_scale, out=out)
         if self.bias is not None:

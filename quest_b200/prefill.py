@@ -103,29 +103,43 @@ class Block(nn.Module):
 
     def forward_fused(self, x, table):
         """The same block with every quantiser fused into the producer of its input: RMSNorm -> quantise is one kernel
-        (its result feeds c_attn, and w1 and w2 share one quantisation), SiLU(w1 x) * w2 x -> quantise is one kernel.
+        (its result feeds c_attn, and w1 and w2 share one quantisation; the second one adds the residual, too),
+        SiLU(w1 x) * w2 x -> quantise is one kernel, and q and k are rotated where the projection has left them.
         Needs W4A4 linears with the Hadamard transform (swap_linears(..., 'int4_fused'))."""
         B, T, C = x.shape
-
-        def ws(m, k):
-            w = default_cache.get(m, k, x.device, x.dtype)
-            return dict(x_int_packed=w["_a_int_packed"], scale=w["_a_scale"], x_int_row_sum=w["_a_int_row_sum"])
-
         flat = x.reshape(-1, C)
-        q = quest.rmsnorm_hadamard_quantize_int4(flat, self.ln_1.weight, self.ln_1.eps, HADAMARD_BLOCK, **ws(flat.size(0), C))
+        m, ffn = flat.size(0), self.mlp.w1.out_features
+
+        def ws(k, n):  # codes (int8 operand or packed), scales and row sums for a linear with k inputs and n outputs
+            w = default_cache.get(m, k, x.device, x.dtype, int8_operand=k % HADAMARD_BLOCK == 0 and quest.layer_operand(m, k, n))
+            return dict(codes=w["_a_int8"] if "_a_int8" in w else w["_a_int_packed"], scale=w["_a_scale"], x_int_row_sum=w["_a_int_row_sum"])
+
         att = self.attn
-        qkv = att.c_attn.forward_quantized(*q).view(B, T, 3 * C)
-        qh, kh, vh = qkv.split(C, dim=2)
-        qh, kh = apply_rope(qh.view(B, T, att.n_head, -1), kh.view(B, T, att.n_head, -1), table)
-        vh = vh.view(B, T, att.n_head, -1)
+        q = quest.producer_hadamard_quantize(quest.PRODUCE_RMSNORM, flat, norm_weight=self.ln_1.weight, eps=self.ln_1.eps,
+                                             block=HADAMARD_BLOCK, **ws(C, 3 * C))
+        qkv = att.c_attn.forward_quantized(*q)
+        if rope_in_place_ok(qkv, table, T, att.n_head):
+            quest.rope_inplace(qkv, table, T, 2 * C)
+            qh, kh, vh = qkv.view(B, T, 3, att.n_head, -1).unbind(2)
+        else:
+            qh, kh, vh = qkv.view(B, T, 3 * C).split(C, dim=2)
+            qh, kh = apply_rope(qh.view(B, T, att.n_head, -1), kh.view(B, T, att.n_head, -1), table)
+            vh = vh.view(B, T, att.n_head, -1)
         y = F.scaled_dot_product_attention(qh.transpose(1, 2), kh.transpose(1, 2), vh.transpose(1, 2), is_causal=True)
-        x = x + att.c_proj(y.transpose(1, 2).contiguous().view(B, T, C))
-        flat = x.reshape(-1, C)
-        q = quest.rmsnorm_hadamard_quantize_int4(flat, self.ln_2.weight, self.ln_2.eps, HADAMARD_BLOCK, **ws(flat.size(0), C))
+        y = att.c_proj(y.transpose(1, 2).contiguous().view(B, T, C)).view(-1, C)
+        flat, q = quest.add_rmsnorm_hadamard_quantize(flat, y, norm_weight=self.ln_2.weight, eps=self.ln_2.eps,
+                                                      block=HADAMARD_BLOCK, **ws(C, ffn))
         gate = self.mlp.w1.forward_quantized(*q)
         up = self.mlp.w2.forward_quantized(*q)
-        q = quest.silu_mul_hadamard_quantize_int4(gate, up, HADAMARD_BLOCK, **ws(gate.size(0), gate.size(1)))
-        return x + self.mlp.c_proj.forward_quantized(*q).view(B, T, C)
+        q = quest.producer_hadamard_quantize(quest.PRODUCE_SILU_MUL, gate, x2=up, block=HADAMARD_BLOCK, **ws(ffn, C))
+        return (flat + self.mlp.c_proj.forward_quantized(*q)).view(B, T, C)
+
+
+def rope_in_place_ok(qkv: torch.Tensor, table: torch.Tensor, seq: int, n_head: int) -> bool:
+    """Whether ``rope_inplace`` takes these heads and this table (whole 16-byte pieces)."""
+    head = qkv.size(1) // (3 * n_head)
+    return (head % 8 == 0 and qkv.size(1) == 3 * n_head * head and table.dtype in (torch.bfloat16, torch.float32)
+            and table.is_contiguous() and table.size(0) >= seq and 2 * table.size(1) == head and table.data_ptr() % 16 == 0)
 
 
 class Decoder(nn.Module):

@@ -1,0 +1,60 @@
+"""What the fused decoder block adds to the quantisers: the in-place rotary embedding and the residual add in front of the
+norm, against their eager forms, bit for bit."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+import quest_b200 as quest
+from quest_b200.prefill import apply_rope, rope_in_place_ok, rope_table
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("batch,seq,heads,head", [(1, 1, 1, 8), (3, 77, 4, 64), (2, 130, 16, 128)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rope_in_place_equals_the_eager_form(batch, seq, heads, head, dtype):
+    g = torch.Generator(device=DEV).manual_seed(seq)
+    c = heads * head
+    table = rope_table(head, 256).to(DEV).to(dtype)
+    qkv = torch.randn(batch * seq, 3 * c, device=DEV, generator=g).to(torch.bfloat16)
+    q, k, v = (t.reshape(batch, seq, heads, head) for t in qkv.view(batch, seq, 3 * c).split(c, dim=2))
+    q_ref, k_ref = apply_rope(q, k, table)
+    v_ref = v.clone()
+    assert rope_in_place_ok(qkv, table, seq, heads)
+    quest.rope_inplace(qkv, table, seq, 2 * c)
+    got = qkv.view(batch, seq, 3, heads, head)
+    assert got[:, :, 0].equal(q_ref) and got[:, :, 1].equal(k_ref) and got[:, :, 2].equal(v_ref)
+    assert not rope_in_place_ok(qkv, table, 257, heads)
+
+
+@pytest.mark.parametrize("m,k", [(1, 256), (33, 2048), (130, 5632)])
+@pytest.mark.parametrize("block", [64, 128, 256])
+def test_producers_and_residual(m, k, block):
+    g = torch.Generator(device=DEV).manual_seed(m + k)
+    x, y = (torch.randn(m, k, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(k, device=DEV, generator=g)).to(torch.bfloat16)
+
+    def outputs(int8):
+        return (torch.empty(m, k if int8 else k // 2, dtype=torch.uint8, device=DEV), torch.empty(m, 1, dtype=torch.bfloat16, device=DEV),
+                torch.empty(m, 1, dtype=torch.int32, device=DEV))
+
+    def same(got, ref):
+        codes, scale, sums = got
+        if codes.size(1) == k:
+            codes = (codes.view(torch.int8) // 16).view(m, k // 32, 2, 16).transpose(2, 3).reshape(m, k)
+        else:
+            codes = quest.unpack_int4(codes)
+        return codes.equal(quest.unpack_int4(ref[0])) and scale.equal(ref[1]) and sums.equal(ref[2])
+
+    norm = quest.rmsnorm_hadamard_quantize_int4(x, w, 1e-5, block)
+    added = quest.rmsnorm_hadamard_quantize_int4(x + y, w, 1e-5, block)
+    gate = quest.silu_mul_hadamard_quantize_int4(x, y, block)
+    for int8 in (False, True):
+        if int8 and k % 128:
+            continue
+        assert same(quest.producer_hadamard_quantize(quest.PRODUCE_RMSNORM, x, *outputs(int8), norm_weight=w, eps=1e-5, block=block), norm)
+        assert same(quest.producer_hadamard_quantize(quest.PRODUCE_SILU_MUL, x, *outputs(int8), x2=y, block=block), gate)
+        total, got = quest.add_rmsnorm_hadamard_quantize(x, y, w, 1e-5, *outputs(int8), block=block)
+        assert total.equal(x + y) and same(got, added)
