@@ -1806,14 +1806,14 @@ extern "C" int hadamard_quantize_int4_cuda_bf16(void*, void*, void*, const void*
 
 extern "C" int quest_b200_begin_layer(void) {
     const int mask = dependent_launch_mask();
-    tl_layer_mode = true;
+    tl_layer_mode = qb_tl_in_layer = true;
     qb_tl_dependent_quantiser = mask < 0 || (mask & 2) != 0;
     qb_tl_quantiser_kernel = 0;
     return QB200_OK;
 }
 
 extern "C" int quest_b200_end_layer(void) {
-    tl_layer_mode = false;
+    tl_layer_mode = qb_tl_in_layer = false;
     qb_tl_dependent_quantiser = false;
     qb_tl_quantiser_kernel = 0;
     tl_dependent_launch = false;

@@ -111,7 +111,7 @@ hadamard_quant_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const RowPa
     // grid has got here (it waits on the device for this grid's end before it touches anything written here).  Only now
     // that tensor memory is allocated: a dependent block that took it first on a shared SM would wait for this grid
     // while this block waits for the allocation.
-    let_dependents_launch();
+    if (p.let_dependents) let_dependents_launch();
     const int rows_per_tile = P == 1 ? T * nb : nb / P;
     const int unit_rows = P == 1 ? T * nb : nb;  // rows of X2 per unit
 

@@ -17,6 +17,7 @@
 namespace qb {
 
 thread_local bool qb_tl_dependent_quantiser = false;
+thread_local bool qb_tl_in_layer = false;
 thread_local int qb_tl_quantiser_kernel = 0;
 
 struct RowParams {
@@ -37,6 +38,9 @@ struct RowParams {
     int x_out_mode;                // 0 none, 1 transformed values, 2 dequantised values
     int quantize;                  // 0: stop after the scale (find_scale / transform only)
     int row_sum_add;               // row_kernel only: constant added to every row sum
+    int let_dependents;            // inside a layer: the GEMM behind this kernel may be scheduled early.  Never otherwise: what
+                                   // is written here may be the weights of a layer further on, whose GEMM reads its first
+                                   // weights before it waits.
 };
 
 constexpr int kUnit = 1024;        // elements per warp-unit
@@ -126,7 +130,7 @@ __device__ __forceinline__ void hadamard32(float (&f)[32], int lane) {
 // used outputs (dense int8 codes, transformed / dequantised bf16 values).
 template <int HB, int UNITS, bool EXTRAS>
 __global__ void __launch_bounds__(UNITS == 1 ? 256 : 512) row_kernel(const RowParams p) {
-    if (!EXTRAS) let_dependents_launch();  // the GEMM of a layer without the transform; it waits for this grid itself
+    if (!EXTRAS && p.let_dependents) let_dependents_launch();
     const int row = blockIdx.x;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -381,9 +385,9 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
         atomicMax(&g_hq_trace[1], t);
     }
 #endif
-    // A kernel launched behind this one with a programmatic dependency (the small-M GEMM of the fused layer call) may
-    // start its own prologue now; it waits for this grid's results itself.  Without such a dependent this does nothing.
-    let_dependents_launch();
+    // A kernel launched behind this one with a programmatic dependency (the GEMM of the layer call) may start its own
+    // prologue now; it waits for this grid's results itself.
+    if (p.let_dependents) let_dependents_launch();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int grp = warp / W;      // row group of this warp
@@ -1085,6 +1089,7 @@ extern "C" int hadamard_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* sc
     p.M = batch_size;
     p.quantize = 1;
     p.had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)block))));
+    p.let_dependents = qb_tl_in_layer;
     if (!vector_path_ok(p)) return QB200_ERR_UNSUPPORTED;
     // Tensor-core kernel where the shape fits its tiling; QB200_HQ_KERNEL=mma|tc forces one (tests, tuning).
     const char* force = getenv("QB200_HQ_KERNEL");
@@ -1225,6 +1230,7 @@ extern "C" int hadamard_quantize_a8_cuda_bf16(void* a8_ptr, void* scale_ptr, voi
     p.quantize = 1;
     p.had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)block))));
     if (!hq_tc_eligible(p, block)) return QB200_ERR_UNSUPPORTED;
+    p.let_dependents = qb_tl_in_layer;
     qb_tl_quantiser_kernel = kQuantiserTc;
     switch (block) {
         case 64: return launch_hq_tc<64>(p, stream);
@@ -1248,6 +1254,7 @@ int quantise_layer_operand(void* a8, void* scale, void* row_sum, const void* x, 
     p.K = K;
     p.M = M;
     p.quantize = 1;
+    p.let_dependents = qb_tl_in_layer;
     if (!vector_path_ok(p)) return QB200_ERR_UNSUPPORTED;
     if (block == 0) {
         qb_tl_quantiser_kernel = kQuantiserMma;
