@@ -197,12 +197,16 @@ int quest_b200_prefers_a8(int M, int K, int N);
 int quest_b200_layer_operand(int M, int K, int N);
 
 /*
- * The layer in one call with or without (block 0) the Hadamard transform, on packed codes ([M, K/2]) or, with int8_operand,
- * on the int8 operand ([M, K]): what quest_b200.layer.linear_forward calls.
+ * The layer in one call with or without (block 0) the Hadamard transform, on packed codes ([M, K/2]; int8_operand 0), on the
+ * int8 operand ([M, K]; 1), or as one kernel that needs no codes, scales and row sums (2; they may be NULL): what
+ * quest_b200.layer.linear_forward calls.  quest_b200_layer_plan returns the fastest of the three for a shape.  bias (bf16 [N], may be NULL) is added to the
+ * bf16 result as a separate add would, where quest_b200_layer_adds_bias returns 1 (QB200_ERR_UNSUPPORTED elsewhere).
  */
 int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add, const void* w_scale,
-                           void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M, int K, int N, int block,
-                           cudaStream_t stream);
+                           const void* bias, void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M, int K,
+                           int N, int block, cudaStream_t stream);
+int quest_b200_layer_plan(int M, int K, int N, int block);
+int quest_b200_layer_adds_bias(int M, int K, int N, int int8_operand);
 
 /*
  * Fused block-Hadamard + scale + int4 quantise + pack + row-sum of bf16 activations, one pass over
@@ -313,6 +317,10 @@ int rope_inplace_cuda_bf16(void* x, const void* table, int table_is_bf16, int ro
 int producer_hadamard_quantize_cuda_bf16(void* codes_ptr, int int8_operand, void* scale_ptr, void* x_int_row_sum_ptr, int producer,
                                          const void* x_ptr, const void* x2_ptr, void* sum_ptr, const void* norm_weight_ptr,
                                          float eps, int group_size, int batch_size, int block, cudaStream_t stream);
+
+/* y = bf16(bf16(x * rsqrt(mean(x^2) + eps)) * weight) per row (src/models/llama.py:64-76).  group_size a multiple of 8,
+ * pointers 16-byte aligned (QB200_ERR_UNSUPPORTED otherwise). */
+int rmsnorm_cuda_bf16(void* y, const void* x, const void* weight, float eps, int group_size, int batch_size, cudaStream_t stream);
 
 #ifdef __cplusplus
 }

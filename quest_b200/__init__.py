@@ -480,6 +480,17 @@ def one_pass_ok(x: torch.Tensor, weight_block: int = 0) -> bool:
             and (weight_block == 0 or weight_block in (64, 128, 256) and x.size(1) % weight_block == 0) and x.data_ptr() % 16 == 0)
 
 
+def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+    """(x.float() * rsqrt(mean(x^2) + eps)).type_as(x) * weight over the last dimension in one kernel (bf16)."""
+    assert x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.is_contiguous() and weight.is_contiguous()
+    k = x.size(-1)
+    assert weight.numel() == k
+    y = torch.empty_like(x)
+    dev = _lib.require_cuda(x, weight)
+    _call("rmsnorm_cuda_bf16", dev, _lib.ptr(y), _lib.ptr(x), _lib.ptr(weight), float(eps), k, x.numel() // k if k else 0, _lib.stream_of(x))
+    return y
+
+
 def rope_inplace(x: torch.Tensor, table: torch.Tensor, seq: int, cols: int) -> torch.Tensor:
     """Rotates the heads in the first ``cols`` columns of x [rows, ld] bf16 in place; row r is position r % seq of ``table``
     (length, head_dim/2, 2), fp32 or bf16.  The same bits as the eager form of src/models/llama.py:43-62."""

@@ -33,12 +33,15 @@ SIGNATURES = {
     "fused_matmul_dequantize_a8_int4t_bf16_cuda": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _P],
     "quest_b200_prefers_a8": [_I, _I, _I],
     "quest_b200_layer_operand": [_I, _I, _I],
-    "w4a4_linear_layer_cuda": [_P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "w4a4_linear_layer_cuda": [_P, _P, _P, _P, _P, _P, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "quest_b200_layer_plan": [_I, _I, _I, _I],
+    "quest_b200_layer_adds_bias": [_I, _I, _I, _I],
     "quest_b200_copy_block_to_peers_cuda": [_P, ctypes.POINTER(ctypes.c_void_p), _I, _I, _I, _LL, _P],
     "quest_b200_begin_layer": [],
     "quest_b200_end_layer": [],
     "hadamard_transform_cuda_bf16": [_P, _P, _I, _I, _I, _I, _P],
     "scale_quantize_int4_cuda_bf16": [_P, _P, _P, _P, _I, _I, _I, _I, _P],
+    "rmsnorm_cuda_bf16": [_P, _P, _P, ctypes.c_float, _I, _I, _P],
     "rope_inplace_cuda_bf16": [_P, _P, _I, _I, _I, _I, _I, _LL, _P],
     "producer_hadamard_quantize_cuda_bf16": [_P, _I, _P, _P, _I, _P, _P, _P, _P, ctypes.c_float, _I, _I, _I, _P],
     "quest_b200_test_bounded_wait_cuda": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _LL, _P],

@@ -29,6 +29,7 @@
 #include <string.h>
 #include <type_traits>
 
+#include "hadamard_unit.cuh"
 #include "tcgen05.cuh"
 
 // Set (per host thread) by the one-call layer entry points around their GEMM call: the GEMM kernel is then launched
@@ -109,6 +110,7 @@ struct EpilogueParams {
     int slab_ints;          // slab_rows * 256: a slab holds only the rows a tile can have (M rounded up to 8, at most 128)
     int* counters;          // one per output tile, all zero between launches
     int tma_store;          // 256 x 256 kernel, fused: the output tensor map is valid (the last tile leaves as bulk tensor stores)
+    const __nv_bfloat16* bias;  // [N] or null (fused; pair, few-token and dp4a kernels): added to the bf16 result, which is rounded again
     int test_skip_producer; // tests only: the TMA producer issues nothing, so that every bounded wait of the launch runs out
     // 256-row kernel: the N range is cut into col_count tile columns whose widths are multiples of 16, at most 256; the
     // first col_rem of them are (col_units + 1) * 16 wide, the others col_units * 16 (col_units = 16, col_rem = 0: all 256)
@@ -149,31 +151,45 @@ __device__ __forceinline__ void dequant_chunk(const uint32_t (&r)[32], int a_add
     }
 }
 
+// y += bias on 32 bf16 results of one row, with the two roundings of the separate add.
+__device__ __forceinline__ void add_bias_chunk(uint32_t (&w)[16], const float* sb_bias) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float2 b = *reinterpret_cast<const float2*>(sb_bias + 2 * i);
+        w[i] = pack_bf16x2(bf16lo_to_f32(w[i]) + b.x, bf16hi_to_f32(w[i]) + b.y);
+    }
+}
+
+// 32 bf16 results of one row -> global memory, clipped to N.
+__device__ __forceinline__ void store_bf16_chunk(const uint32_t (&w)[16], const EpilogueParams& ep, int row, int col0, int N) {
+    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld + col0;
+    if (ep.vec_ok == 2 && col0 + 32 <= N) {
+        stg256(out, w);
+        stg256(out + 16, w + 8);
+        return;
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        const int col = col0 + 8 * g;
+        if (ep.vec_ok && col + 8 <= N) {
+            *reinterpret_cast<uint4*>(out + 8 * g) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (col + i < N)
+                    reinterpret_cast<uint16_t*>(out)[8 * g + i] = (uint16_t)(w[4 * g + i / 2] >> (16 * (i & 1)));
+        }
+    }
+}
+
 template <bool FUSED>
 __device__ __forceinline__ void epilogue_store_chunk(const uint32_t (&r)[32], const EpilogueParams& ep, int row, int col0,
                                                      int N, int a_add, float half_a_mul, const int* sb_add,
                                                      const float* sb_mul) {
     if (FUSED) {
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(ep.out) + (size_t)row * ep.ld + col0;
         uint32_t w[16];  // the 32 results as bf16 pairs
         dequant_chunk(r, a_add, half_a_mul, sb_add, sb_mul, w);
-        if (ep.vec_ok == 2 && col0 + 32 <= N) {
-            stg256(out, w);
-            stg256(out + 16, w + 8);
-        } else {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                const int col = col0 + 8 * g;
-                if (ep.vec_ok && col + 8 <= N) {
-                    *reinterpret_cast<uint4*>(out + 8 * g) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (col + i < N)
-                            reinterpret_cast<uint16_t*>(out)[8 * g + i] = (uint16_t)(w[4 * g + i / 2] >> (16 * (i & 1)));
-                }
-            }
-        }
+        store_bf16_chunk(w, ep, row, col0, N);
     } else {
         int32_t* out = static_cast<int32_t*>(ep.out) + (size_t)row * ep.ld + col0;
         if (ep.vec_ok == 2 && col0 + 32 <= N) {
@@ -1644,8 +1660,9 @@ using namespace qb;
 //    GEMM is launched behind it: -1 ... -2 us per layer;
 //  * below that the quantiser is the small CUDA-core kernel in plain stream order and only the GEMM is dependent (its
 //    set-up and first weight requests overlap the quantiser): -1.5 us per layer at M = 64 ... 512, K = 4096;
-//  * a GEMM launched that way behind the CUDA-core quantiser of a large input measured slower (+1 ... +10 us at 4 M
-//    elements and more), so where the tcgen05 kernel cannot tile K both launches stay plain.
+//  * behind the CUDA-core quantiser of a large input the GEMM may be scheduled when the quantiser's blocks have done
+//    their last rows, not when they start: its waiting blocks would take their place (+1 ... +10 us at 4 M elements and
+//    more).
 // QB200_DEPENDENT_LAUNCH in the environment (tests, tuning) forces the launches instead: bit 0 = the GEMM, bit 1 = the
 // quantiser is launched with a programmatic dependency; 0 = both in plain stream order.
 static thread_local bool tl_layer_mode = false;
@@ -1656,18 +1673,29 @@ static int dependent_launch_mask() {
 }
 
 // Before a GEMM launch: inside a layer the kernel before it in the stream is the layer's quantiser.
-static void note_layer_launch(int M, int K) {
+static void note_layer_launch() {
     if (!tl_layer_mode) return;
     const int mask = dependent_launch_mask();
-    const bool small = (long long)M * K < 3ll * 1024 * 1024;
-    tl_dependent_launch = mask >= 0 ? (mask & 1) != 0
-                                    : (qb_tl_quantiser_kernel == kQuantiserTc || (qb_tl_quantiser_kernel == kQuantiserMma && small));
+    tl_dependent_launch = mask >= 0 ? (mask & 1) != 0 : qb_tl_quantiser_kernel != 0;
     qb_tl_quantiser_kernel = 0;  // consumed: a second GEMM of the layer follows a GEMM, not the quantiser
+}
+
+static int run_gemm_a8(const EpilogueParams& ep_in, const void* mat_a8, const void* mat_b, int M, int K, int N, cudaStream_t stream) {
+    EpilogueParams ep = ep_in;
+    ep.vec_ok = aligned16(ep.out) && (ep.ld % 8 == 0);
+    if (ep.vec_ok && (reinterpret_cast<uintptr_t>(ep.out) & 31u) == 0 && ep.ld % 16 == 0) ep.vec_ok = 2;
+    int dev = 0;
+    const int sms = sm_count_of_current_device(&dev);
+    if (sms < 2) return QB200_ERR_CUDA;
+    note_layer_launch();
+    const int st = launch_gemm_a8(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
+    tl_dependent_launch = false;
+    return st;
 }
 
 static int run_gemm(bool fused, const EpilogueParams& ep, const void* a, const void* b, int M, int K, int N,
                     cudaStream_t stream, int static_splits = -1) {
-    note_layer_launch(M, K);
+    note_layer_launch();
     const int st = run_gemm_impl(fused, ep, a, b, M, K, N, stream, static_splits);
     tl_dependent_launch = false;
     return st;
@@ -1734,18 +1762,9 @@ extern "C" int fused_matmul_dequantize_a8_int4t_bf16_cuda(void* mat_d, const voi
     ep.b_add = static_cast<const int32_t*>(vec_b_add);
     ep.a_mul = static_cast<const __nv_bfloat16*>(vec_a_mul);
     ep.b_mul = static_cast<const __nv_bfloat16*>(vec_b_mul);
-    ep.vec_ok = aligned16(mat_d) && (N % 8 == 0);
-    if (ep.vec_ok && (reinterpret_cast<uintptr_t>(mat_d) & 31u) == 0 && N % 16 == 0) ep.vec_ok = 2;
-    int dev = 0;
-    const int sms = sm_count_of_current_device(&dev);
-    if (sms <= 0) return QB200_ERR_CUDA;
-    note_layer_launch(M, K);
-    const int st = launch_gemm_a8(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
-    tl_dependent_launch = false;
-    return st;
+    return run_gemm_a8(ep, mat_a8, mat_b, M, K, N, stream);
 }
 
-constexpr int kGemvRows = 4;  // of a layer; provisional
 constexpr bool kA8ByDefault = true;  // measured faster wherever the 256 x 256 kernel and the tcgen05 quantiser both apply (QB200_A8=0 switches it off)
 
 // 1 if, for this layer shape, the int8-operand route (hadamard_quantize_a8_cuda_bf16 + the GEMM above) is the faster one:
@@ -1775,7 +1794,10 @@ extern "C" int quest_b200_layer_operand(int M, int K, int N) {
     int dev = 0;
     const int sms = sm_count_of_current_device(&dev);
     if (sms < 2) return 0;
-    return M > kGemvRows || !gemv_eligible(M, K, N, 0);
+    // Up to two rows the dp4a kernel on packed codes streams the weights faster (layer, M 2: K 8192 N 10240 13.0 against
+    // 15.5 us, K 11008 N 4096 10.2 / 11.5; M 3: 17.1 / 15.5, 12.5 / 11.5), except for a long K with few weight rows, which
+    // leave it too few warps (M 1 K 28672 N 1024: 20.4 / 14.8).
+    return M > 2 || !gemv_eligible(M, K, N, 0) || (K > 16384 && N < 4096);
 }
 
 extern "C" int fused_matmul_dequantize_int4_int4t_bf16_noalloc_cuda(void* mat_d, const void* mat_a, const void* mat_b,
@@ -1848,19 +1870,52 @@ extern "C" int w4a4_linear_hadamard_a8_bf16_cuda(void* mat_d, const void* x, con
 
 extern "C" int scale_quantize_int4_cuda_bf16(void*, void*, void*, const void*, int, int, int, int, cudaStream_t);
 
+// How a layer that is free to choose runs: 0 packed codes, 1 int8 operand, 2 one kernel (no workspace at all).
+extern "C" int quest_b200_layer_plan(int M, int K, int N, int block) {
+    int per;
+    if (M > 0 && N > 0 && K > 0 && getenv("QB200_GEMM_TILE") == nullptr && getenv("QB200_GEMM_SPLITS") == nullptr &&
+        getenv("QB200_GEMM_GEMV") == nullptr && getenv("QB200_A8") == nullptr && getenv("QB200_HQ_KERNEL") == nullptr &&
+        gemv_layer_parts(M, K, N, block, &per) > 0)
+        return 2;
+    return quest_b200_layer_operand(M, K, N);
+}
+
+// The layer: quantiser, then GEMM.  bias: only where quest_b200_layer_adds_bias says so.
+extern "C" int quest_b200_layer_adds_bias(int M, int K, int N, int int8_operand) {
+    return int8_operand ? 1 : (getenv("QB200_GEMM_TILE") == nullptr && getenv("QB200_GEMM_SPLITS") == nullptr &&
+                               getenv("QB200_GEMM_GEMV") == nullptr && gemv_eligible(M, K, N, 0));
+}
+
 extern "C" int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add, const void* w_scale,
-                                      void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M, int K, int N,
-                                      int block, cudaStream_t stream) {
-    if (block != 0)
-        return int8_operand ? w4a4_linear_hadamard_a8_bf16_cuda(mat_d, x, w_int_packed, w_add, w_scale, codes, a_scale, a_int_row_sum, M, K, N, block, stream)
-                            : w4a4_linear_hadamard_bf16_cuda(mat_d, x, w_int_packed, w_add, w_scale, codes, a_scale, a_int_row_sum, M, K, N, block, stream);
-    if (!a_int_row_sum) return QB200_ERR_INVALID_ARGUMENT;
+                                      const void* bias, void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M,
+                                      int K, int N, int block, cudaStream_t stream) {
+    if (M < 0 || N < 0 || K < 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (M == 0 || N == 0) return QB200_OK;
+    if (!mat_d || !x || !w_int_packed || !w_add || !w_scale) return QB200_ERR_INVALID_ARGUMENT;
+    if (int8_operand != 2 && (!codes || !a_scale || !a_int_row_sum)) return QB200_ERR_INVALID_ARGUMENT;
+    if (K == 0 || K % (int8_operand == 1 ? 128 : 32) != 0 || K >= (1 << 17)) return QB200_ERR_UNSUPPORTED;
+    if (!aligned16(x) || !aligned16(codes) || !aligned16(w_int_packed)) return QB200_ERR_INVALID_ARGUMENT;
+    if (bias && !quest_b200_layer_adds_bias(M, K, N, int8_operand)) return QB200_ERR_UNSUPPORTED;
+    EpilogueParams ep{};
+    ep.out = mat_d;
+    ep.ld = N;
+    ep.a_add = static_cast<const int32_t*>(a_int_row_sum);
+    ep.b_add = static_cast<const int32_t*>(w_add);
+    ep.a_mul = static_cast<const __nv_bfloat16*>(a_scale);
+    ep.b_mul = static_cast<const __nv_bfloat16*>(w_scale);
+    ep.bias = static_cast<const __nv_bfloat16*>(bias);
+    if (int8_operand == 2) {
+        int dev = 0;
+        const int sms = sm_count_of_current_device(&dev);
+        if (sms <= 0) return QB200_ERR_CUDA;
+        return run_gemv_layer(ep, x, w_int_packed, M, K, N, block, sms, dev, stream);
+    }
     quest_b200_begin_layer();
-    int st = int8_operand ? quantise_layer_operand(codes, a_scale, a_int_row_sum, x, K, M, 0, stream)
+    int st = int8_operand ? quantise_layer_operand(codes, a_scale, a_int_row_sum, x, K, M, block, stream)
+             : block != 0 ? hadamard_quantize_int4_cuda_bf16(codes, a_scale, a_int_row_sum, x, K, M, block, stream)
                           : scale_quantize_int4_cuda_bf16(codes, a_scale, a_int_row_sum, x, K, M, 0, 0, stream);
     if (st == QB200_OK)
-        st = int8_operand ? fused_matmul_dequantize_a8_int4t_bf16_cuda(mat_d, codes, w_int_packed, a_int_row_sum, w_add, a_scale, w_scale, M, K, N, stream)
-                          : fused_matmul_dequantize_int4_int4t_bf16_cuda(mat_d, codes, w_int_packed, a_int_row_sum, w_add, a_scale, w_scale, M, K, N, stream);
+        st = int8_operand ? run_gemm_a8(ep, codes, w_int_packed, M, K, N, stream) : run_gemm(true, ep, codes, w_int_packed, M, K, N, stream);
     quest_b200_end_layer();
     return st;
 }

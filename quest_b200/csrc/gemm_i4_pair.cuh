@@ -36,7 +36,7 @@ constexpr int kWarps = kAWarp + 1;
 constexpr int kThreads = kWarps * 32;
 constexpr int SLAB_BYTES = 32 * 64;            // one output piece: 32 rows x 32 columns of bf16
 constexpr int SLABS_BYTES = kEpiWarps * SLAB_BYTES;
-constexpr int VEC_STRIDE = TN * 8;             // per accumulator buffer: b_add (int32) and b_mul (fp32) of the tile
+constexpr int VEC_STRIDE = TN * 12;            // per accumulator buffer: b_add (int32), b_mul and bias (fp32) of the tile
 constexpr int NUM_BARS = 2 * P_STAGES + 2 * STAGES + 4 + 1;
 constexpr int LAYOUT_BYTES = STAGES * STAGE_BYTES + P_STAGES * P_BYTES + SLABS_BYTES + 2 * VEC_STRIDE + NUM_BARS * 8 + 16;
 constexpr int SMEM_BYTES = LAYOUT_BYTES + 1024;
@@ -240,10 +240,12 @@ gemm_i4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             const bool row_ok = row < M;
             int* sb_add = reinterpret_cast<int*>(smem_raw + (vec_base - raw_base) + acc * VEC_STRIDE);
             float* sb_mul = reinterpret_cast<float*>(sb_add + TN);
+            float* sb_bias = sb_mul + TN;
             {
                 const bool in = et < bn && n0 + et < N;
                 sb_add[et] = in ? ep.b_add[n0 + et] : 0;
                 sb_mul[et] = in ? bf16_to_f32(ep.b_mul[n0 + et]) : 0.f;
+                if (ep.bias != nullptr) sb_bias[et] = in ? bf16_to_f32(ep.bias[n0 + et]) : 0.f;
             }
             int a_add = 0;
             float half_a_mul = 0.f;
@@ -266,12 +268,13 @@ gemm_i4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 uint32_t r[32];
                 tmem_ld32(t_row + c0, r);
                 tmem_ld_wait32(r);
-                if (!ep.tma_store) {
-                    if (row_ok) epilogue_store_chunk<true>(r, ep, row, n0 + c0, N, a_add, half_a_mul, sb_add + c0, sb_mul + c0);
-                    continue;
-                }
                 uint32_t w[16];
                 dequant_chunk(r, a_add, half_a_mul, sb_add + c0, sb_mul + c0, w);
+                if (ep.bias != nullptr) add_bias_chunk(w, sb_bias + c0);
+                if (!ep.tma_store) {
+                    if (row_ok) store_bf16_chunk(w, ep, row, n0 + c0, N);
+                    continue;
+                }
                 const uint32_t slab = last ? ring_slab + (uint32_t)(pc - first) * SLAB_BYTES : own_slab;
                 if (!last) {
                     if (lane == 0) bulk_wait_read_all();  // the previous piece has left the slab

@@ -236,12 +236,13 @@ gemm_i4_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const int c = lane * 4;
     if (c < rows) {
         int ba[4];
-        float bm[4];
+        float bm[4], bias[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const bool in = n0 + c + i < N;
             ba[i] = in ? ep.b_add[n0 + c + i] : 0;
             bm[i] = in ? bf16_to_f32(ep.b_mul[n0 + c + i]) : 0.f;
+            bias[i] = in && ep.bias != nullptr ? bf16_to_f32(ep.bias[n0 + c + i]) : 0.f;
         }
         for (int m = rank + warp * S; m < M; m += kWarps * S) {
             const uint32_t src = smem_base + (uint32_t)(m * W_ROWS + c) * 4u;
@@ -263,7 +264,11 @@ gemm_i4_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
 #pragma unroll
             for (int i = 0; i < 4; ++i) v[i] = (float)((acc[i] >> 7) + a_add + ba[i]) * (am * bm[i]);
             __nv_bfloat16* out = static_cast<__nv_bfloat16*>(ep.out) + (size_t)m * ep.ld + n0 + c;
-            const uint32_t w0 = pack_bf16x2(v[0], v[1]), w1 = pack_bf16x2(v[2], v[3]);
+            uint32_t w0 = pack_bf16x2(v[0], v[1]), w1 = pack_bf16x2(v[2], v[3]);
+            if (ep.bias != nullptr) {
+                w0 = pack_bf16x2(bf16lo_to_f32(w0) + bias[0], bf16hi_to_f32(w0) + bias[1]);
+                w1 = pack_bf16x2(bf16lo_to_f32(w1) + bias[2], bf16hi_to_f32(w1) + bias[3]);
+            }
             if (vec && n0 + c + 4 <= N) {
                 *reinterpret_cast<uint2*>(out) = make_uint2(w0, w1);
             } else {

@@ -12,6 +12,7 @@
 //   two rounding points decide the codes - the Hadamard output is rounded to bf16 before anything
 //   else looks at it, and the scale is rounded to bf16 before the divide.
 #include "common.cuh"
+#include "hadamard_unit.cuh"
 #include "tcgen05.cuh"
 
 namespace qb {
@@ -19,6 +20,8 @@ namespace qb {
 thread_local bool qb_tl_dependent_quantiser = false;
 thread_local bool qb_tl_in_layer = false;
 thread_local int qb_tl_quantiser_kernel = 0;
+
+constexpr long long kTcFromInLayer = 3ll * 1024 * 1024;  // elements; see the crossover at hadamard_quantize_int4_cuda_bf16
 
 struct RowParams {
     const __nv_bfloat16* x;        // [M,K] input
@@ -38,16 +41,13 @@ struct RowParams {
     int x_out_mode;                // 0 none, 1 transformed values, 2 dequantised values
     int quantize;                  // 0: stop after the scale (find_scale / transform only)
     int row_sum_add;               // row_kernel only: constant added to every row sum
-    int let_dependents;            // inside a layer: the GEMM behind this kernel may be scheduled early.  Never otherwise: what
+    int let_dependents;            // inside a layer: the GEMM behind this kernel may be scheduled early (1: at once, 2: when a
+                                   // block has done its last rows; mma.sync kernel only).  Never otherwise: what
                                    // is written here may be the weights of a layer further on, whose GEMM reads its first
                                    // weights before it waits.
 };
 
-constexpr int kUnit = 1024;        // elements per warp-unit
 constexpr int kMaxVectorK = 64 * kUnit;  // 16 warps x 4 units; longer rows take the scalar kernel
-constexpr float kFloorMagic = 12582912.0f;  // 1.5 * 2^23: adding it (round-down) leaves floor(y) in the low mantissa bits
-constexpr int kFloorMagicBits = 0x4B400000;
-
 // floor(x / s) for bf16-valued x and s, without a divide.
 //
 // x / s is an exact integer for about 1 % of the elements, so a plain x * (1/s) mis-floors.  For
@@ -63,35 +63,11 @@ __device__ __forceinline__ int floor_quotient(float x, float inv_s) {
     return __float_as_int(__fadd_rd(y2, kFloorMagic)) - kFloorMagicBits;
 }
 
-// Same as floor_quotient but returns the raw bits of the magic-number sum: for |x/s| < 2^22 the low bits are
-// floor(x/s) in two's complement, so for a pre-clamped x the low nibble is the int4 code.
-__device__ __forceinline__ uint32_t floor_quotient_bits(float x, float inv_s) {
-    const float y = x * inv_s;
-    const float y2 = fmaf(fabsf(y), 1.220703125e-4f, y);
-    return __float_as_uint(__fadd_rd(y2, kFloorMagic));
-}
-
-// Element-wise clamp of a bf16 pair to [lo, hi] (both given as bf16 pairs).
-__device__ __forceinline__ uint32_t clamp_bf16x2(uint32_t v, uint32_t lo, uint32_t hi) {
-    uint32_t r;
-    asm("{\n\t.reg .b32 t;\n\tmax.bf16x2 t, %1, %2;\n\tmin.bf16x2 %0, t, %3;\n\t}" : "=r"(r) : "r"(v), "r"(lo), "r"(hi));
-    return r;
-}
-
 // (sat4(a) << 4 | sat4(b)) | (c << 8): saturating pack of two int32 to signed nibbles.
 __device__ __forceinline__ uint32_t pack_sat_s4(int hi, int lo, uint32_t c) {
     uint32_t d;
     asm("cvt.pack.sat.s4.s32.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(hi), "r"(lo), "r"(c));
     return d;
-}
-
-// Sum of the eight signed nibbles of w, times 16, accumulated into acc.
-__device__ __forceinline__ int nibble_sum16(uint32_t w, int acc) {
-    const uint32_t lo = (w << 4) & 0xF0F0F0F0u;
-    const uint32_t hi = w & 0xF0F0F0F0u;
-    acc = __dp4a((int)lo, 0x01010101, acc);
-    acc = __dp4a((int)hi, 0x01010101, acc);
-    return acc;
 }
 
 // 32 packed codes as the GEMM's int8 operand: sixteen times the codes, the even positions of the group first (see q_a8).
@@ -305,29 +281,9 @@ __global__ void __launch_bounds__(UNITS == 1 ? 256 : 512) row_kernel(const RowPa
 //   butterflies, round to bf16 pairs (kept in registers until the row's scale is known)
 //   quantise -> 2-byte pieces -> warp-private shared staging -> one coalesced 16-byte store per lane.
 // -------------------------------------------------------------------------------------------------
-constexpr int kBlkPitch = 272;              // 256-byte block of 128 bf16 + 16 bytes of padding
-constexpr int kStepIn = 8 * kBlkPitch;      // eight blocks per warp step
-constexpr int kOutPitch = 80;               // 64 packed bytes per block + 16 bytes of padding
 constexpr int kMaxDynSmem = 220 * 1024;  // leaves room for the static reduction arrays under the 227 KB limit
 constexpr int kStepBytes = 2 * kStepIn;  // two input buffers (the next row is prefetched); the packed codes are
                                          // staged in the buffer that has just been consumed
-
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool valid) {
-    const int sz = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(sz) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
 
 // Thread-block shape: G row groups x W warps.  The W warps of a group share one row (UNITS 1024-element
 // units per warp); the block walks over batches of G rows.  Everything that is per row rather than per
@@ -344,20 +300,6 @@ __device__ __forceinline__ unsigned long long hq_gtime() {
 }
 #endif
 
-// Packed fp32 pairs (sm_100 executes add/sub/mul/fma on two floats per instruction).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpk2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 add2_rd(f32x2 a, f32x2 b) { f32x2 r; asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-
 // PRO: what produces the rows that are transformed and quantised.
 //   0  the input itself.
 //   1  RMSNorm of the input:  y = bf16( bf16(x * rsqrt(mean(x^2) + eps)) * w )   (src/models/llama.py:64-76: the
@@ -369,6 +311,30 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm(
 // The producer rewrites the row in shared memory, in place, between the copy and the tensor-core stage; everything
 // after it is unchanged.  It saves the producer's own kernel(s), one write and one read of [M, K] bf16.
 constexpr int kProNone = 0, kProRmsNorm = 1, kProSiluMul = 2, kProAddRmsNorm = 3;
+
+// silu of eight bf16 values, rounded to bf16 as the correctly rounded fp32 quotient x / (1 + exp(-x)) is: the product with
+// the approximate reciprocal is within 3 ulp of the quotient, which matters only within 4 ulp of a tie between two bf16
+// values (one in 7000); there, and for divisors whose reciprocal comes near the subnormal range, the chunk is divided in
+// full.  One branch per eight values.
+__device__ __forceinline__ void silu8(const uint32_t (&w)[4], uint32_t (&t)[4]) {
+    float d[8], q[8];
+    bool exact = false;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float a = (i & 1) ? bf16hi_to_f32(w[i / 2]) : bf16lo_to_f32(w[i / 2]);
+        d[i] = 1.f + expf(-a);
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d[i]));  // d >= 1
+        q[i] = a * r;
+        exact |= (__float_as_uint(q[i]) & 0xFFFFu) - 0x7FFCu <= 8u || !(d[i] < 1e30f);
+    }
+    if (exact) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q[i] = __fdiv_rn((i & 1) ? bf16hi_to_f32(w[i / 2]) : bf16lo_to_f32(w[i / 2]), d[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t[i] = pack_bf16x2(q[2 * i], q[2 * i + 1]);
+}
 
 template <int HB, int UNITS, int PRO = kProNone>
 __global__ void __launch_bounds__(256, UNITS == 1 ? 4 : (UNITS == 2 ? 3 : 2))
@@ -387,7 +353,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
 #endif
     // A kernel launched behind this one with a programmatic dependency (the GEMM of the layer call) may start its own
     // prologue now; it waits for this grid's results itself.
-    if (p.let_dependents) let_dependents_launch();
+    if (p.let_dependents == 1) let_dependents_launch();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int grp = warp / W;      // row group of this warp
@@ -426,20 +392,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
 
     // ---- B fragments: h * H16[k][o], MMA column n of tile nu is output o = 4*(n>>1) + 2*nu + (n&1) ----
     uint32_t bfrag[2][2];
-    {
-        const uint32_t hb = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(p.had_scale));
-#pragma unroll
-        for (int nu = 0; nu < 2; ++nu) {
-            const int o = 4 * (g >> 1) + 2 * nu + (g & 1);
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int k0 = 2 * tig + 8 * half;
-                const uint32_t lo = hb | ((__popc(k0 & o) & 1) ? 0x8000u : 0u);
-                const uint32_t hi = hb | ((__popc((k0 + 1) & o) & 1) ? 0x8000u : 0u);
-                bfrag[nu][half] = lo | (hi << 16);
-            }
-        }
-    }
+    hadamard16_fragments(p.had_scale, lane, bfrag);
 
     int prev_batch = -1, last_par = 0;
     for (int it = 0; batch < num_batches; batch += gridDim.x, ++it) {
@@ -464,6 +417,14 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
 #pragma unroll
                 for (int u = 0; u < UNITS; ++u) {
                     const uint32_t in_base = smem_w + u * step_bytes + buf * kStepIn;
+                    uint4 in2[4];
+                    if (PRO == kProAddRmsNorm) {  // a unit's pieces are requested together
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int e = (u * W + wig) * kUnit + (j * 32 + lane) * 8;
+                            if (e < K && row < M) in2[j] = *reinterpret_cast<const uint4*>(p.x2 + (size_t)row * K + e);
+                        }
+                    }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int c = j * 32 + lane;
@@ -472,7 +433,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
                         uint32_t w4[4] = {q.x, q.y, q.z, q.w};
                         const int e = (u * W + wig) * kUnit + c * 8;
                         if (PRO == kProAddRmsNorm && e < K && row < M) {
-                            const uint4 o = *reinterpret_cast<const uint4*>(p.x2 + (size_t)row * K + e);
+                            const uint4 o = in2[j];
                             const uint32_t o4[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
                             for (int i = 0; i < 4; ++i)
@@ -505,6 +466,14 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
             for (int u = 0; u < UNITS; ++u) {
                 const int unit = u * W + wig;
                 const uint32_t in_base = smem_w + u * step_bytes + buf * kStepIn;
+                uint4 in2[4];
+                if (PRO == kProSiluMul) {  // a unit's pieces are requested together, before the first is used
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int e = unit * kUnit + (j * 32 + lane) * 8;
+                        if (e < K && row_p < M) in2[j] = ld_stream16(p.x2 + (size_t)row_p * K + e);
+                    }
+                }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int c = j * 32 + lane;
@@ -512,23 +481,18 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
                     if (e >= K || row_p >= M) continue;
                     const uint32_t addr = in_base + (c >> 4) * kBlkPitch + (c & 15) * 16;
                     const uint4 q = lds128(addr);
-                    const uint4 o = kNorm ? __ldg(reinterpret_cast<const uint4*>(p.norm_w + e))
-                                                       : ld_stream16(p.x2 + (size_t)row_p * K + e);
+                    const uint4 o = kNorm ? __ldg(reinterpret_cast<const uint4*>(p.norm_w + e)) : in2[j];
                     const uint32_t w4[4] = {q.x, q.y, q.z, q.w}, o4[4] = {o.x, o.y, o.z, o.w};
-                    uint32_t y4[4];
+                    uint32_t t4[4], y4[4];  // t4: the producer's first rounding to the activation type
+                    if (kNorm) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        float a = bf16lo_to_f32(w4[i]), b = bf16hi_to_f32(w4[i]);
-                        if (kNorm) {
-                            a *= rinv;
-                            b *= rinv;
-                        } else {
-                            a = __fdiv_rn(a, 1.f + expf(-a));
-                            b = __fdiv_rn(b, 1.f + expf(-b));
-                        }
-                        const uint32_t t = pack_bf16x2(a, b);  // the producer's first rounding to the activation type
-                        y4[i] = pack_bf16x2(bf16lo_to_f32(t) * bf16lo_to_f32(o4[i]), bf16hi_to_f32(t) * bf16hi_to_f32(o4[i]));
+                        for (int i = 0; i < 4; ++i) t4[i] = pack_bf16x2(bf16lo_to_f32(w4[i]) * rinv, bf16hi_to_f32(w4[i]) * rinv);
+                    } else {
+                        silu8(w4, t4);
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        y4[i] = pack_bf16x2(bf16lo_to_f32(t4[i]) * bf16lo_to_f32(o4[i]), bf16hi_to_f32(t4[i]) * bf16hi_to_f32(o4[i]));
                     sts128(addr, make_uint4(y4[0], y4[1], y4[2], y4[3]));
                 }
             }
@@ -539,61 +503,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
         f32x2 ssq2 = 0ull;
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
-            const uint32_t in_base = smem_w + u * step_bytes + buf * kStepIn;
-            f32x2 f[8][2];  // f[a][h]: elements 16a + 4tig + 2h, +1 of block g, as packed float pairs
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                uint32_t a[4];
-                ldmatrix_x4(in_base + (lane & 7) * kBlkPitch + (2 * t + ((lane >> 3) & 1)) * 32 + (lane >> 4) * 16, a);
-#pragma unroll
-                for (int nu = 0; nu < 2; ++nu) {
-                    float d[4];
-                    mma_bf16_16816(d, a, bfrag[nu][0], bfrag[nu][1]);
-                    f[2 * t][nu] = pk2(d[0], d[1]);
-                    f[2 * t + 1][nu] = pk2(d[2], d[3]);
-                }
-            }
-            // remaining index bits 4.. of the block: butterflies over the row index a (in registers)
-#pragma unroll
-            for (int s = 1; s < 8 && s < HB / 16; s <<= 1) {
-#pragma unroll
-                for (int a = 0; a < 8; ++a) {
-                    if ((a & s) == 0) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const f32x2 x0 = f[a][h], x1 = f[a + s][h];
-                            f[a][h] = add2(x0, x1);
-                            f[a + s][h] = sub2(x0, x1);
-                        }
-                    }
-                }
-            }
-            if (HB == 256) {  // index bit 7 pairs neighbouring 128-element halves: lanes g and g ^ 1
-                const float sgn = (g & 1) ? -1.f : 1.f;
-#pragma unroll
-                for (int a = 0; a < 8; ++a)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        float x0, x1;
-                        unpk2(f[a][h], x0, x1);
-                        const float p0 = __shfl_xor_sync(0xffffffffu, x0, 4);
-                        const float p1 = __shfl_xor_sync(0xffffffffu, x1, 4);
-                        f[a][h] = pk2(fmaf(x0, sgn, p0), fmaf(x1, sgn, p1));
-                    }
-            }
-#pragma unroll
-            for (int a = 0; a < 8; ++a)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    float x0, x1;
-                    unpk2(f[a][h], x0, x1);
-                    v[u][2 * a + h] = pack_bf16x2(x0, x1);
-                }
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const f32x2 xx = pk2(bf16lo_to_f32(v[u][i]), bf16hi_to_f32(v[u][i]));
-                ssq2 = fma2(xx, xx, ssq2);
-            }
+            transform_unit<HB>(smem_w + u * step_bytes + buf * kStepIn, lane, bfrag, v[u], ssq2);
         }
         float ssq;
         {
@@ -613,15 +523,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
         double tot = 0.0;
         for (int i = 0; i < W; ++i) tot += (double)part_ssq[par][grp * W + i];
         const __nv_bfloat16 sb = __float2bfloat16_rn(quest_scale_from_mean_square(__fdiv_rn((float)tot, (float)K)));
-        const float s_f = bf16_to_f32(sb);
-        const float inv_s = __frcp_rn(s_f);
-        // Saturation is done on the bf16 pairs before the divide: x is clamped to [-8s, ~7.5s], both bounds
-        // exact or safely inside [7s, 8s), so floor(x/s) lands in [-8, 7] without integer min/max, and the
-        // code is simply the low nibble of the magic-number sum.
-        const uint32_t lo1 = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(-8.f * s_f));
-        const uint32_t hi1 = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(7.5f * s_f));
-        const uint32_t lo2 = lo1 | (lo1 << 16), hi2 = hi1 | (hi1 << 16);
-        const f32x2 inv_s2 = pk2(inv_s, inv_s), magic2 = pk2(kFloorMagic, kFloorMagic);
+        const RowConstants rc = row_constants(sb);
         if (wig == 0 && lane == 0 && row < M) p.scale_out[row] = sb;
         if (warp == 0 && lane < G && prev_batch >= 0 && p.row_sum != nullptr) {
             const int pr = prev_batch * G + lane;
@@ -639,41 +541,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
         for (int u = 0; u < UNITS; ++u) {
             const int unit = u * W + wig;
             const uint32_t out_base = smem_w + u * step_bytes + buf * kStepIn;  // input already consumed
-#pragma unroll
-            for (int pr = 0; pr < 4; ++pr) {  // rows a = 2pr and 2pr + 1: eight codes -> one 32-bit word
-                uint32_t ub[8];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t c = clamp_bf16x2(v[u][4 * pr + i], lo2, hi2);
-                    float y0, y1;
-                    unpk2(mul2(pk2(bf16lo_to_f32(c), bf16hi_to_f32(c)), inv_s2), y0, y1);
-                    // nudge towards +inf by |y| * 2^-13 (see floor_quotient), then floor through the magic-number sum
-                    const f32x2 fl = add2_rd(pk2(fmaf(fabsf(y0), 1.220703125e-4f, y0), fmaf(fabsf(y1), 1.220703125e-4f, y1)), magic2);
-                    float u0, u1;
-                    unpk2(fl, u0, u1);
-                    ub[2 * i] = __float_as_uint(u0);
-                    ub[2 * i + 1] = __float_as_uint(u1);
-                }
-                // ub[0..3] = row 2pr elements 0..3, ub[4..7] = row 2pr+1 elements 0..3; code = low nibble
-                const uint32_t ev = __byte_perm(__byte_perm(ub[0], ub[2], 0x0040), __byte_perm(ub[4], ub[6], 0x0040), 0x5410);
-                const uint32_t od = __byte_perm(__byte_perm(ub[1], ub[3], 0x0040), __byte_perm(ub[5], ub[7], 0x0040), 0x5410);
-                const uint32_t word = (ev & 0x0F0F0F0Fu) | ((od << 4) & 0xF0F0F0F0u);
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(out_base + g * kOutPitch + pr * 16 + tig * 4), "r"(word) : "memory");
-            }
-            __syncwarp();
-            uint4 t4;  // lane reads rows (2c, 2c+1) of block lane>>2, c = lane&3: one word per source thread tig
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                         : "=r"(t4.x), "=r"(t4.y), "=r"(t4.z), "=r"(t4.w) : "r"(out_base + (lane >> 2) * kOutPitch + (lane & 3) * 16));
-            __syncwarp();  // the staging area is rewritten for the next row
-            uint4 w;   // low halves are row 2c (bytes 2tig, 2tig+1), high halves row 2c+1
-            w.x = __byte_perm(t4.x, t4.y, 0x5410);
-            w.y = __byte_perm(t4.z, t4.w, 0x5410);
-            w.z = __byte_perm(t4.x, t4.y, 0x7632);
-            w.w = __byte_perm(t4.z, t4.w, 0x7632);
-            rs16 = nibble_sum16(w.x, rs16);
-            rs16 = nibble_sum16(w.y, rs16);
-            rs16 = nibble_sum16(w.z, rs16);
-            rs16 = nibble_sum16(w.w, rs16);
+            const uint4 w = quantise_unit(v[u], rc, out_base, lane, rs16);
             const int e0 = unit * kUnit + lane * 32;
             if (row < M && p.q_a8 != nullptr) {  // K is a multiple of 128 here
                 if (e0 < K) store_a8(p.q_a8 + (size_t)row * K + e0, w);
@@ -696,6 +564,7 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
         last_par = par;
     }
     // row sums of the last batch
+    if (p.let_dependents == 2) let_dependents_launch();
     __syncthreads();
 #ifdef QB200_TRACE
     if (threadIdx.x == 0) {
@@ -718,7 +587,9 @@ template <int HB, bool EXTRAS>
 static int launch_row(const RowParams& p, cudaStream_t stream);
 
 template <int HB, int PRO = kProNone>
-static int launch_hq_mma(const RowParams& p, cudaStream_t stream) {
+static int launch_hq_mma(const RowParams& p_in, cudaStream_t stream) {
+    RowParams p = p_in;
+    if (p.let_dependents && (long long)p.M * p.K >= kTcFromInLayer) p.let_dependents = 2;
     const int units = (p.K + kUnit - 1) / kUnit;
     // units per warp, warps per row, rows per block (at most 16 warps per block)
     int per = units >= 2 ? 2 : 1;  // two units per warp amortise the per-row work best (measured)
@@ -979,6 +850,55 @@ __global__ void copy_block_kernel(const uint8_t* __restrict__ src, const CopyDst
     }
 }
 
+// RMSNorm of bf16 rows, y = bf16(bf16(x * rsqrt(mean x^2 + eps)) * w): one warp per row, the row read once into registers
+// in pieces of 2048 elements (longer rows are read a second time, from L1 or L2).  HBM-bound, 4 bytes per element.
+__global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x,
+                                                      const __nv_bfloat16* __restrict__ w, const int M, const int K, const float eps) {
+    const int lane = threadIdx.x & 31;
+    for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < M; row += gridDim.x * 8) {
+        const __nv_bfloat16* xr = x + (size_t)row * K;
+        uint4 held[8];
+        float sum = 0.f;
+        for (int base = 0; base < K; base += 2048) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int e = base + (j * 32 + lane) * 8;
+                held[j] = e < K ? *reinterpret_cast<const uint4*>(xr + e) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint32_t v[4] = {held[j].x, held[j].y, held[j].z, held[j].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float a = bf16lo_to_f32(v[i]), b = bf16hi_to_f32(v[i]);
+                    sum = fmaf(a, a, sum);
+                    sum = fmaf(b, b, sum);
+                }
+            }
+        }
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        const float rinv = rsqrtf(__fdiv_rn(sum, (float)K) + eps);
+        for (int base = 0; base < K; base += 2048) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int e = base + (j * 32 + lane) * 8;
+                if (e >= K) continue;
+                if (K > 2048) held[j] = *reinterpret_cast<const uint4*>(xr + e);
+                const uint4 wv = __ldg(reinterpret_cast<const uint4*>(w + e));
+                const uint32_t v[4] = {held[j].x, held[j].y, held[j].z, held[j].w}, u[4] = {wv.x, wv.y, wv.z, wv.w};
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t t = pack_bf16x2(bf16lo_to_f32(v[i]) * rinv, bf16hi_to_f32(v[i]) * rinv);
+                    o[i] = pack_bf16x2(bf16lo_to_f32(t) * bf16lo_to_f32(u[i]), bf16hi_to_f32(t) * bf16hi_to_f32(u[i]));
+                }
+                *reinterpret_cast<uint4*>(y + (size_t)row * K + e) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        }
+    }
+}
+
 // -------------------------------------------------------------------------------------------------
 // Rotary embedding of q and k where the fused projection has left them (columns [0, cols) of each qkv row), in place.
 // HBM-bound: one read and one write of q and k, 4 bytes per element, against a dozen passes in fp32 of the eager form.
@@ -1069,7 +989,6 @@ extern "C" int quantize_int4_cuda_bf16(void* x_ptr, const void* scale_ptr, void*
     return run_rows(p, 0, extras, stream);
 }
 
-constexpr long long kTcFromInLayer = 3ll * 1024 * 1024;  // see the crossover below
 
 extern "C" int hadamard_quantize_int4_cuda_bf16(void* x_int_packed_ptr, void* scale_ptr, void* x_int_row_sum_ptr,
                                                 const void* x_ptr, int group_size, int batch_size, int block,
@@ -1334,6 +1253,18 @@ extern "C" int add_mul_vv_cuda_bf16(void* mat_d, const void* vec_a_add, const vo
         add_mul_vv_vec8_kernel<<<(unsigned)blocks, 256, 0, stream>>>(d, aa, am, ba, bm, c, size_a, size_b);
     else
         add_mul_vv_scalar_kernel<<<(unsigned)blocks, 256, 0, stream>>>(d, aa, am, ba, bm, c, size_a, size_b);
+    return launch_status();
+}
+
+extern "C" int rmsnorm_cuda_bf16(void* y, const void* x, const void* weight, float eps, int group_size, int batch_size, cudaStream_t stream) {
+    if (group_size < 0 || batch_size < 0) return QB200_ERR_INVALID_ARGUMENT;
+    if (group_size == 0 || batch_size == 0) return QB200_OK;
+    if (!y || !x || !weight) return QB200_ERR_INVALID_ARGUMENT;
+    if (group_size % 8 != 0 || !aligned16(y) || !aligned16(x) || !aligned16(weight)) return QB200_ERR_UNSUPPORTED;
+    int blocks = (batch_size + 7) / 8;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    rmsnorm_kernel<<<blocks, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(x),
+                                               static_cast<const __nv_bfloat16*>(weight), batch_size, group_size, eps);
     return launch_status();
 }
 

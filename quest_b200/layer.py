@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 import quest_b200 as quest
 from . import _lib
@@ -91,10 +92,11 @@ def _one_call_ok(*tensors: torch.Tensor) -> bool:
 _BLOCKS = (64, 128, 256)
 
 
-def _layer_call(x, w, w_scale, w_add, out, ws, block):
+def _layer_call(x, w, w_scale, w_add, out, ws, block, bias=None):
     """The whole layer as one library call, or None where its buffers are not what that call takes (linear_forward then goes
     through the single ops, which check and report).  ``block`` 0: no transform.  ``ws``: None, or (codes, scale, row sums)
-    where codes [M, K] selects the int8 operand and [M, K/2] packed int4; None takes one allocation for all three."""
+    where codes [M, K] selects the int8 operand and [M, K/2] packed int4; None takes one allocation for all three.
+    ``bias``: added as ``y += bias`` would, in the GEMM's epilogue where it can."""
     if x.dim() != 2 or w.dim() != 2 or not x.is_cuda:
         return None
     (m, k), n, dev = x.shape, w.size(0), x.get_device()
@@ -108,17 +110,20 @@ def _layer_call(x, w, w_scale, w_add, out, ws, block):
     if xp % 16 or wp % 16:
         return None
     if out is None:
-        out = torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
+        out = x.new_empty((m, n))
     elif out.shape != (m, n) or out.dtype is not torch.bfloat16 or out.get_device() != dev or not out.is_contiguous():
         return None
     lib = _lib.load()
     if ws is None:
-        int8 = lib.quest_b200_layer_operand(m, k, n)
-        code_bytes = -(-(m * k if int8 else m * (k // 2)) // 256) * 256
-        buf = torch.empty(code_bytes + 6 * m, dtype=torch.uint8, device=x.device)
-        codes = buf.data_ptr()
-        sums = codes + code_bytes
-        scale = sums + 4 * m
+        int8 = lib.quest_b200_layer_plan(m, k, n, block)
+        if int8 == 2:  # one kernel, no workspace
+            codes = sums = scale = None
+        else:
+            code_bytes = -(-(m * k if int8 else m * (k // 2)) // 256) * 256
+            buf = x.new_empty(code_bytes // 2 + 3 * m)  # bf16 elements: two bytes each
+            codes = buf.data_ptr()
+            sums = codes + code_bytes
+            scale = sums + 4 * m
     else:
         a, a_scale, a_sums = ws
         if (a.shape not in ((m, k), (m, k // 2)) or a.dtype is not torch.uint8 or a_scale.dtype is not torch.bfloat16
@@ -128,9 +133,13 @@ def _layer_call(x, w, w_scale, w_add, out, ws, block):
             return None
         int8 = int(a.size(1) == k)
         codes, scale, sums = a.data_ptr(), a_scale.data_ptr(), a_sums.data_ptr()
-    if int8 and k % 128:
+    if int8 == 1 and k % 128:
         return None
-    args = (out.data_ptr(), xp, wp, w_add.data_ptr(), w_scale.data_ptr(), codes, int8, scale, sums, m, k, n, block,
+    late_bias = None  # a bias that autograd follows is added by torch
+    if bias is not None and not (not (bias.requires_grad and torch.is_grad_enabled()) and forward_ad._current_level < 0 and bias.dtype is torch.bfloat16 and bias.dim() == 1 and bias.size(0) == n and bias.get_device() == dev
+                                 and bias.is_contiguous() and lib.quest_b200_layer_adds_bias(m, k, n, int8)):
+        bias, late_bias = None, bias
+    args = (out.data_ptr(), xp, wp, w_add.data_ptr(), w_scale.data_ptr(), None if bias is None else bias.data_ptr(), codes, int8, scale, sums, m, k, n, block,
             torch._C._cuda_getCurrentRawStream(dev))
     if torch._C._cuda_getDevice() == dev:
         status = lib.w4a4_linear_layer_cuda(*args)
@@ -139,6 +148,8 @@ def _layer_call(x, w, w_scale, w_add, out, ws, block):
             status = lib.w4a4_linear_layer_cuda(*args)
     if status:
         _lib.check(status, "w4a4_linear_layer_cuda")
+    if late_bias is not None:
+        out += late_bias
     return out
 
 
@@ -271,11 +282,20 @@ class Linear4bit(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not self.use_noop:
-            a = x.contiguous().flatten(end_dim=-2)
+            a = x.contiguous()
+            if a.dim() != 2:
+                a = a.flatten(end_dim=-2)
             # activation-side workspaces come from the shared per-stream cache: nothing but the output is allocated
             m, k = a.shape
-            a8 = quest.layer_operand(m, k, self.out_features)
-            ws = self.workspaces.get(m, k, a.device, a.dtype, int8_operand=a8)
+            block = HADAMARD_BLOCK if self.use_hadamard else 0
+            plan = _lib.load().quest_b200_layer_plan(m, k, self.out_features, block)
+            ws, buffers = {}, None
+            if plan != 2:
+                ws = self.workspaces.get(m, k, a.device, a.dtype, int8_operand=plan == 1)
+                buffers = (ws["_a_int8"] if plan == 1 else ws["_a_int_packed"], ws["_a_scale"], ws["_a_int_row_sum"])
+            y = _layer_call(a, self.w_int_packed, self.w_scale, self.w_add, None, buffers, block, self.bias)
+            if y is not None:
+                return y if x.dim() == 2 else y.view(*x.shape[:-1], self.out_features)
             y = linear_forward(activation=a, w_int_packed=self.w_int_packed, w_scale=self.w_scale, w_add=self.w_add,
                                w_meta_e=self.w_meta_e, out=None, use_hadamard=self.use_hadamard, **ws)
             y = y.unflatten(dim=0, sizes=x.shape[:-1])

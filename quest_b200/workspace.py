@@ -20,7 +20,7 @@ class WorkspaceCache:
     def get(self, m: int, k: int, device: torch.device, dtype: torch.dtype = torch.bfloat16, int8_operand: bool = False) -> dict:
         """{'_a_scale': [M,1] dtype, '_a_int_row_sum': [M,1] int32, and '_a_int_packed': [M,K/2] uint8 or, with
         ``int8_operand``, '_a_int8': [M,K] uint8} for the current stream of ``device``."""
-        stream = torch.cuda.current_stream(device).cuda_stream
+        stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
         key = (device.index, stream, m, k, dtype, bool(int8_operand))
         ws = self._sets.get(key)
         if ws is None:

@@ -58,3 +58,31 @@ def test_producers_and_residual(m, k, block):
         assert same(quest.producer_hadamard_quantize(quest.PRODUCE_SILU_MUL, x, *outputs(int8), x2=y, block=block), gate)
         total, got = quest.add_rmsnorm_hadamard_quantize(x, y, w, 1e-5, *outputs(int8), block=block)
         assert total.equal(x + y) and same(got, added)
+
+
+@pytest.mark.parametrize("m,k", [(1, 8), (37, 2048), (9, 2056), (5, 5632)])
+def test_rmsnorm_kernel(m, k):
+    g = torch.Generator(device=DEV).manual_seed(k)
+    x = torch.randn(m, k, device=DEV, generator=g).to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(k, device=DEV, generator=g)).to(torch.bfloat16)
+    y = quest.rmsnorm(x, w, 1e-5)
+    xd = x.double()
+    exact = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    # two roundings to bf16: the significand has 8 bits, half an ulp is at most 2^-8 of the value
+    assert (y.double() - exact).abs().le(2 * 2.0 ** -8 * exact.abs() * 1.01 + 1e-30).all()
+
+
+def test_silu_quotient_keeps_every_rounding():
+    """The gate of the fused quantiser against torch's silu over all bf16 values: the block is quantised with a scale that
+    the gate itself decides, so every value is put alone into a row of its own next to a fixed one."""
+    bits = torch.arange(65536, device=DEV, dtype=torch.int32).to(torch.int16)
+    vals = bits.view(torch.bfloat16)
+    vals = vals[vals.isfinite()]
+    gate = torch.zeros(vals.numel(), 64, dtype=torch.bfloat16, device=DEV)
+    gate[:, 0] = vals
+    up = torch.ones_like(gate)
+    ref = quest.hadamard_quantize_int4(torch.nn.functional.silu(gate) * up, 64)
+    got = quest.silu_mul_hadamard_quantize_int4(gate, up, 64)
+    ok = torch.isfinite(ref[1].flatten())
+    # the row's scale is a function of silu(v) alone, monotone in its magnitude: a gate rounded the other way moves it
+    assert got[1].flatten()[ok].equal(ref[1].flatten()[ok])

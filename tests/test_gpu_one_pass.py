@@ -18,6 +18,8 @@ def test_one_pass_equals_the_separate_ops(rows, k, block):
     g = torch.Generator(device=DEV).manual_seed(rows + k)
     x = (torch.randn(rows, k, device=DEV, generator=g) * torch.rand(rows, 1, device=DEV, generator=g)).to(torch.bfloat16)
     x[0, : k // 2] = 0
+    x[0, : k // 4] = -0.0
+    x[rows - 1, k // 2:] *= 1e-6  # quotients far below one, of both signs, beside full-sized ones
     before = x.clone()
     assert quest.one_pass_ok(x, block)
     packed, scale, sums = quest.scale_quantize_int4(x, weight_block=block, row_sum_add=k // 2)
