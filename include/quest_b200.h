@@ -179,8 +179,7 @@ int fused_matmul_dequantize_int4_int4t_bf16_push_cuda(void* const* mat_d_list, i
  * row-major, and inside every group of 32 consecutive K positions the 16 even positions first, then the 16 odd
  * ones - so that the GEMM need not unpack A.  Only shapes the tcgen05 quantiser can tile (group_size a multiple of
  * 128, see quest_b200_prefers_a8); QB200_ERR_UNSUPPORTED otherwise.  fused_matmul_dequantize_a8_int4t_bf16_cuda is the
- * fused GEMM + epilogue taking that operand (mat_b stays packed int4; K a multiple of 128; always the 256 x 256 tile
- * kernel).  quest_b200_prefers_a8 returns 1 where this route is the faster one for an [M, K] x [N, K]^T layer (what
+ * fused GEMM + epilogue taking that operand (mat_b stays packed int4; K a multiple of 128).  quest_b200_prefers_a8 returns 1 where this route is the faster one for an [M, K] x [N, K]^T layer (what
  * quest_b200.layer.linear_forward asks before choosing), else 0; QB200_A8=0|1 in the environment overrides it.
  */
 int hadamard_quantize_a8_cuda_bf16(void* a8_ptr, void* scale_ptr, void* x_int_row_sum_ptr, const void* x_ptr,

@@ -1369,15 +1369,18 @@ struct SkinnyPlan {
 // Weight rows per CTA and K ranges of the skinny kernel, in cycles.  Measured (K = 4096, N = 11008 and 12288): a step of
 // 128 K takes 440 / 475 / 565 / 720 cycles of an SM at 16 / 32 / 64 / 128 tokens whatever the weight rows are (the issue
 // of four MMAs, then the tokens' way through shared memory), a launch about 8000 cycles, the exchange of a cluster 2500
-// and each wave of CTAs beyond the first about 3000.
+// and each wave of CTAs beyond the first about 3000.  Larger clusters do not reach every SM: with one CTA per SM, clusters
+// of four and eight leave 16 and 28 of 148 SMs without one (the occupancy calculator's count; with splits of three and
+// more estimated on 144 SMs, M 81 K 2048 N 6144 took 18.6 instead of 13.3 us).
 static SkinnyPlan pick_skinny(int tn, int K, int N, int sms) {
     const int num_kb = K / BK;
     const int per_sm = tn <= 32 ? 2 : 1;
     const long long step = tn <= 16 ? 440 : (tn <= 32 ? 475 : (tn <= 64 ? 565 : 720));
     SkinnyPlan best{0, 0, -1};
-    for (int s = 1; s <= skinny::kMaxSplit && s <= num_kb; ++s) {
-        // SMs that clusters of this size can use: the GPU's SMs come in groups of 16 to 20
-        const int usable = s <= 2 ? sms : sms - sms % 16;
+    for (int s = 1; s <= skinny::kMaxSplit && s <= num_kb; s *= 2) {
+        int usable = sms;
+        if (s > 2) usable = per_sm == 2 ? sms - 4 : (s == 4 ? sms - 16 : sms - 28);
+        if (usable < s) continue;
         for (int rows = skinny::W_ROWS; rows >= 8; rows -= 8) {
             const long long ctas = (long long)((N + rows - 1) / rows) * s;
             const long long waves = (ctas + (long long)usable * per_sm - 1) / ((long long)usable * per_sm);
@@ -1438,7 +1441,8 @@ static long long pair_cycles(int M, int K, int N, int sms) {
 // kernel elsewhere.  QB200_A8_KERNEL=pair|skinny forces one (tests, tuning).
 static int launch_gemm_a8(const EpilogueParams& ep, const void* a8, const void* b, int M, int K, int N, int sms, int dev,
                           cudaStream_t stream) {
-    bool use_skinny = M <= 128 && pick_skinny(skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms);
+    // Up to 32 rows the skinny kernel whatever the estimates say: seven eighths of a pair's rows would be empty.
+    bool use_skinny = M <= 32 || (M <= 128 && pick_skinny(skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms));
     if (const char* e = getenv("QB200_A8_KERNEL")) use_skinny = e[0] == 's' && M <= 128;
     if (!use_skinny) return launch_gemm_pair(ep, a8, b, M, K, N, sms, dev, stream);
     switch (skinny_tokens(M)) {
@@ -1794,10 +1798,12 @@ extern "C" int quest_b200_layer_operand(int M, int K, int N) {
     int dev = 0;
     const int sms = sm_count_of_current_device(&dev);
     if (sms < 2) return 0;
-    // Up to two rows the dp4a kernel on packed codes streams the weights faster (layer, M 2: K 8192 N 10240 13.0 against
-    // 15.5 us, K 11008 N 4096 10.2 / 11.5; M 3: 17.1 / 15.5, 12.5 / 11.5), except for a long K with few weight rows, which
-    // leave it too few warps (M 1 K 28672 N 1024: 20.4 / 14.8).
-    return M > 2 || !gemv_eligible(M, K, N, 0) || (K > 16384 && N < 4096);
+    // For a few rows the dp4a kernel on packed codes streams the weights faster (layer, packed / int8, M 2: K 8192 N 10240
+    // 13.0 / 15.5 us; M 4: K 8192 N 3584 9.7 / 12.3; M 3: K 8192 N 10240 17.1 / 15.5, K 11008 N 4096 12.5 / 11.5), except
+    // for a long K with few weight rows, which leave it too few warps (M 1 K 28672 N 1024: 20.4 / 14.8).
+    if (gemv_eligible(M, K, N, 0) && (M <= 2 || (M <= 4 && (long long)M * N * K <= 120000000ll)) && !(K > 16384 && N < 4096)) return 0;
+    // A narrow layer on a large input pays for the operand's second byte: M 7008 K 28672 N 1024 261 against 271 us.
+    return (long long)M * K <= (48ll << 20) || N >= 1536;
 }
 
 extern "C" int fused_matmul_dequantize_int4_int4t_bf16_noalloc_cuda(void* mat_d, const void* mat_a, const void* mat_b,

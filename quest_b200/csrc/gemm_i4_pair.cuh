@@ -119,13 +119,14 @@ gemm_i4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         }
     }
     __syncwarp();
+    cluster_sync();  // both CTAs have started and initialised their barriers: an allocation for the pair involves the other CTA
     if (warp == 1) {
         tmem_alloc_pair(tmem_slot, 512);
         tmem_relinquish_pair();
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync();  // both CTAs' barriers are initialised and their tensor memory is allocated
+    cluster_sync();  // tensor memory is allocated in both
     tc_fence_after();
     const uint32_t tmem_acc = *tmem_slot_ptr;
     let_dependents_launch();  // only now that tensor memory is allocated (see gemm_i4_kernel)
@@ -350,4 +351,5 @@ gemm_i4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after();
         tmem_dealloc_pair(tmem_acc, 512);
     }
+    cluster_sync();  // neither CTA leaves before the other has released the pair's tensor memory
 }

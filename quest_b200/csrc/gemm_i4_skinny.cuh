@@ -146,6 +146,7 @@ gemm_i4_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         if (elect_one()) umma_commit(done);  // on a give-up, too: the commit covers whatever was issued
         __syncwarp();
         mbar_wait(done, 0, 55);
+        __syncwarp();
     } else if (warp == kTokenWarp) {
         // ------------------------------ token producer ------------------------------
         if (lane == 0) {
