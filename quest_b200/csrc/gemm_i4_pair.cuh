@@ -311,7 +311,12 @@ gemm_i4_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 if ((int)(it & 1u) != grp) continue;
                 const uint32_t ps = it % P_STAGES, pph = (it / P_STAGES) & 1u;
                 const uint32_t us = it % STAGES, uph = (it / STAGES) & 1u;
-                ok = mbar_wait(full_p + 8 * ps, pph, 38) && mbar_wait(empty + 8 * us, uph ^ 1u, 39);
+                // The operand stage first: the MMAs of step it - STAGES have then completed, so every copy up to that step has
+                // landed, slot ps is in the phase this step waits for, and its parity names only that one.  The other way
+                // round nothing has ended the slot's use before, which was the OTHER group's (P_STAGES is odd): a late copy
+                // leaves the barrier a phase behind, whose parity is the same, and the wait returns at once.
+                static_assert(STAGES <= P_STAGES, "a packed slot's use before this one has ended");
+                ok = mbar_wait(empty + 8 * us, uph ^ 1u, 39) && mbar_wait(full_p + 8 * ps, pph, 38);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 const uint32_t src = p_base + ps * P_BYTES;

@@ -173,6 +173,9 @@ gemm_i4_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         for (int it = grp; it < steps; it += 2) {
             const uint32_t ps = (uint32_t)it % C::P_STAGES, pph = ((uint32_t)it / C::P_STAGES) & 1u;
             const uint32_t us = (uint32_t)it % C::U_STAGES, uph = ((uint32_t)it / C::U_STAGES) & 1u;
+            // The parity of full_p names one phase only if the slot's use before (step it - P_STAGES) has ended: on an even ring
+            // it was this group's own, on an odd one the MMAs of step it - 2 - U_STAGES, which this group has waited for, say so.
+            static_assert(C::P_STAGES % 2 == 0 || C::U_STAGES + 2 <= C::P_STAGES, "a packed slot's use before this one has ended");
             bool ok = mbar_wait(full_p + 8 * ps, pph, 56) && mbar_wait(empty + 8 * us, uph ^ 1u, 57);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;

@@ -52,6 +52,20 @@ def test_pair_kernel(monkeypatch, m, k, n):
     check(args, want)
 
 
+# long reductions over many columns: over a hundred steps of the packed ring, the weights from HBM (their copies land out of
+# order when memory is cold: nine sets of weights larger than L2 together take turns)
+@pytest.mark.parametrize("m,k,n", [(33, 28672, 776), (130, 28672, 2048), (300, 16384, 4096), (256, 28672, 8192)])
+def test_pair_kernel_long_reductions(monkeypatch, m, k, n):
+    monkeypatch.setenv("QB200_A8_KERNEL", "pair")
+    (a8, w, a_add, b_add, a_mul, b_mul), want = problem(m, k, n, m + k + n)
+    turns = [(torch.roll(w, i, 0), torch.roll(b_add, i, 0), torch.roll(b_mul, i, 0)) for i in range(9)]
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+    for _ in range(3):
+        flush.zero_()
+        for i, (wi, add, mul) in enumerate(turns):
+            check((a8, wi, a_add, add, a_mul, mul), torch.roll(want, i, 1))
+
+
 def test_pair_and_few_token_kernels_at_the_largest_sums(monkeypatch):
     for kernel, m in (("pair", 130), ("skinny", 16)):
         monkeypatch.setenv("QB200_A8_KERNEL", kernel)
