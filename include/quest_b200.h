@@ -200,6 +200,7 @@ int quest_b200_layer_operand(int M, int K, int N);
  * int8 operand ([M, K]; 1), or as one kernel that needs no codes, scales and row sums (2; they may be NULL): what
  * quest_b200.layer.linear_forward calls.  quest_b200_layer_plan returns the fastest of the three for a shape.  bias (bf16 [N], may be NULL) is added to the
  * bf16 result as a separate add would, where quest_b200_layer_adds_bias returns 1 (QB200_ERR_UNSUPPORTED elsewhere).
+ * QB200_ERR_UNSUPPORTED for a block other than 0, 64, 128 or 256, and for block 0 in the one-kernel form.
  */
 int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add, const void* w_scale,
                            const void* bias, void* codes, int int8_operand, void* a_scale, void* a_int_row_sum, int M, int K,

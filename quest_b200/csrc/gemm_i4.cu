@@ -1898,7 +1898,9 @@ extern "C" int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_
     if (M < 0 || N < 0 || K < 0) return QB200_ERR_INVALID_ARGUMENT;
     if (M == 0 || N == 0) return QB200_OK;
     if (!mat_d || !x || !w_int_packed || !w_add || !w_scale) return QB200_ERR_INVALID_ARGUMENT;
+    if (int8_operand < 0 || int8_operand > 2) return QB200_ERR_INVALID_ARGUMENT;
     if (int8_operand != 2 && (!codes || !a_scale || !a_int_row_sum)) return QB200_ERR_INVALID_ARGUMENT;
+    if (block != 64 && block != 128 && block != 256 && !(block == 0 && int8_operand != 2)) return QB200_ERR_UNSUPPORTED;
     if (K == 0 || K % (int8_operand == 1 ? 128 : 32) != 0 || K >= (1 << 17)) return QB200_ERR_UNSUPPORTED;
     if (!aligned16(x) || !aligned16(codes) || !aligned16(w_int_packed)) return QB200_ERR_INVALID_ARGUMENT;
     if (bias && !quest_b200_layer_adds_bias(M, K, N, int8_operand)) return QB200_ERR_UNSUPPORTED;

@@ -316,7 +316,8 @@ static int run_gemv_layer(const EpilogueParams& ep, const void* x, const void* b
     switch (block) {
         case 64: return QB_GEMV_LAYER(64);
         case 128: return QB_GEMV_LAYER(128);
-        default: return QB_GEMV_LAYER(256);
+        case 256: return QB_GEMV_LAYER(256);
+        default: return QB200_ERR_UNSUPPORTED;
     }
 #undef QB_GEMV_LAYER
 }

@@ -67,6 +67,13 @@ def test_argument_validation_without_gpu():
     assert lib.quest_b200_copy_block_to_peers_cuda(p, dsts, 2, 4, 60, 64, None) == 2                      # not whole 16-byte pieces
     odd = (ctypes.c_void_p * 2)(p + 256, p + 514)
     assert lib.quest_b200_copy_block_to_peers_cuda(p, odd, 2, 4, 64, 64, None) == 2                       # misaligned destination
+    # the layer refuses a block it has no transform for (the one-kernel form always transforms) and operand forms it has not
+    def layer(operand, block, k=512):
+        return lib.w4a4_linear_layer_cuda(p, p, p, p, p, None, p, operand, p, p, 1, k, 4, block, None)
+    assert [layer(2, b) for b in (0, 32, 96, 512)] == [2] * 4
+    assert [layer(o, b) for o in (0, 1) for b in (32, 512, -1)] == [2] * 6
+    assert layer(3, 128) == 1 and layer(-1, 128) == 1
+    assert layer(1, 0, 96) == 2 and layer(0, 128, 192) == 1 and layer(2, 128, 1 << 17) == 2
     # layer mode is host-thread state: begin / end always succeed and leave the ordinary entry points usable
     assert lib.quest_b200_begin_layer() == 0 and lib.quest_b200_end_layer() == 0
     assert lib.matmul_int4_int4t_int32_cuda(None, None, None, 0, 128, 4, None) == 0
