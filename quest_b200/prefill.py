@@ -15,6 +15,7 @@ import math
 import torch
 import torch.nn.functional as F
 from torch import nn
+from torch.autograd import forward_ad
 
 import quest_b200 as quest
 from .layer import HADAMARD_BLOCK, Linear4bit
@@ -51,6 +52,12 @@ def apply_rope(q: torch.Tensor, k: torch.Tensor, table: torch.Tensor):
     return rot(q), rot(k)
 
 
+def kernels_may_replace(*tensors: torch.Tensor) -> bool:
+    """Whether nothing differentiates through operations of torch on these tensors: no graph is recorded for any of them and no
+    forward-mode level is open.  Only then may a kernel stand in for such an operation (a kernel leaves no graph)."""
+    return forward_ad._current_level < 0 and not (torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float):
         super().__init__()
@@ -59,9 +66,11 @@ class RMSNorm(nn.Module):
         self.fused = False  # one kernel instead of the eager passes, where nothing asks for a graph (swap_linears)
 
     def forward(self, x):
-        if (self.fused and not torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and self.weight.dtype == torch.bfloat16
-                and x.is_contiguous() and x.size(-1) % 8 == 0 and x.data_ptr() % 16 == 0 and self.weight.data_ptr() % 16 == 0):
-            return quest.rmsnorm(x, self.weight, self.eps)
+        w = self.weight
+        if (self.fused and not torch.is_grad_enabled() and kernels_may_replace(x, w) and x.is_cuda and x.dtype == torch.bfloat16
+                and w.dtype == torch.bfloat16 and w.device == x.device and w.shape == x.shape[-1:] and x.is_contiguous()
+                and w.is_contiguous() and x.size(-1) % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
+            return quest.rmsnorm(x, w, self.eps)
         xf = x.float()
         return (xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.eps)).type_as(x) * self.weight
 
@@ -122,7 +131,7 @@ class Block(nn.Module):
         q = quest.producer_hadamard_quantize(quest.PRODUCE_RMSNORM, flat, norm_weight=self.ln_1.weight, eps=self.ln_1.eps,
                                              block=HADAMARD_BLOCK, **ws(C, 3 * C))
         qkv = att.c_attn.forward_quantized(*q)
-        if rope_in_place_ok(qkv, table, T, att.n_head):
+        if kernels_may_replace(qkv, table) and rope_in_place_ok(qkv, table, T, att.n_head):
             quest.rope_inplace(qkv, table, T, 2 * C)
             qh, kh, vh = qkv.view(B, T, 3, att.n_head, -1).unbind(2)
         else:
@@ -131,8 +140,13 @@ class Block(nn.Module):
             vh = vh.view(B, T, att.n_head, -1)
         y = F.scaled_dot_product_attention(qh.transpose(1, 2), kh.transpose(1, 2), vh.transpose(1, 2), is_causal=True)
         y = att.c_proj(y.transpose(1, 2).contiguous().view(B, T, C)).view(-1, C)
-        flat, q = quest.add_rmsnorm_hadamard_quantize(flat, y, norm_weight=self.ln_2.weight, eps=self.ln_2.eps,
-                                                      block=HADAMARD_BLOCK, **ws(C, ffn))
+        if kernels_may_replace(flat, y):
+            flat, q = quest.add_rmsnorm_hadamard_quantize(flat, y, norm_weight=self.ln_2.weight, eps=self.ln_2.eps,
+                                                          block=HADAMARD_BLOCK, **ws(C, ffn))
+        else:  # the residual path is torch's: gradients and tangents pass through it
+            flat = flat + y
+            q = quest.producer_hadamard_quantize(quest.PRODUCE_RMSNORM, flat, norm_weight=self.ln_2.weight, eps=self.ln_2.eps,
+                                                 block=HADAMARD_BLOCK, **ws(C, ffn))
         gate = self.mlp.w1.forward_quantized(*q)
         up = self.mlp.w2.forward_quantized(*q)
         q = quest.producer_hadamard_quantize(quest.PRODUCE_SILU_MUL, gate, x2=up, block=HADAMARD_BLOCK, **ws(ffn, C))

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import quest_b200 as quest
-from quest_b200.prefill import apply_rope, rope_in_place_ok, rope_table
+from quest_b200.prefill import Decoder, DecoderConfig, apply_rope, rope_in_place_ok, rope_table, swap_linears
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -58,6 +58,24 @@ def test_producers_and_residual(m, k, block):
         assert same(quest.producer_hadamard_quantize(quest.PRODUCE_SILU_MUL, x, *outputs(int8), x2=y, block=block), gate)
         total, got = quest.add_rmsnorm_hadamard_quantize(x, y, w, 1e-5, *outputs(int8), block=block)
         assert total.equal(x + y) and same(got, added)
+
+
+def test_fused_block_keeps_the_residual_gradient():
+    torch.manual_seed(1)
+    with torch.device(DEV):
+        model = Decoder(DecoderConfig(n_embd=256, n_layer=2, n_head=4, ffn=512, vocab_size=64, sequence_length=32)).to(torch.bfloat16)
+    swap_linears(model, "int4_fused")
+    x = torch.randn(2, 17, 256, device=DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        ref = [blk(x, model.rope) for blk in model.transformer.h]
+    x.requires_grad_()
+    g = torch.randn_like(x)
+    for blk, y_ref in zip(model.transformer.h, ref):
+        y = blk(x, model.rope)
+        assert y.equal(y_ref)
+        assert torch.autograd.grad(y, x, g)[0].equal(g)
+    model(torch.arange(34, device=DEV).view(2, 17)).float().sum().backward()
+    assert model.transformer.wte.weight.grad.abs().sum() > 0 and model.transformer.ln_f.weight.grad is not None
 
 
 @pytest.mark.parametrize("m,k", [(1, 8), (37, 2048), (9, 2056), (5, 5632)])
