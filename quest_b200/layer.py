@@ -84,12 +84,21 @@ def fused_matmul_dequantize_int4_bf16(
     return mat_d
 
 
-def _one_call_ok(*tensors: torch.Tensor) -> bool:
-    """The one-call layer entry points take dense row-major buffers only."""
-    return all(t.is_contiguous() for t in tensors)
-
-
 _BLOCKS = (64, 128, 256)
+
+
+def _caller_workspaces(x, n, a_int8, a_int_packed, a_scale, a_sums):
+    """(codes, scale, row sums) for ``_layer_call`` from what the caller gave, the missing ones allocated; None if nothing was
+    given.  Of two code buffers the one the library's own choice needs is used."""
+    if a_int8 is None and a_int_packed is None and a_scale is None and a_sums is None:
+        return None
+    m, k = x.shape
+    codes = a_int_packed if a_int8 is None else a_int8
+    if (a_int8 is None) == (a_int_packed is None):
+        int8 = quest.layer_operand(m, k, n)
+        codes = torch.empty(m, k if int8 else k // 2, dtype=torch.uint8, device=x.device) if codes is None else a_int8 if int8 else a_int_packed
+    return (codes, torch.empty(m, 1, dtype=x.dtype, device=x.device) if a_scale is None else a_scale,
+            torch.empty(m, 1, dtype=torch.int32, device=x.device) if a_sums is None else a_sums)
 
 
 def _layer_call(x, w, w_scale, w_add, out, ws, block, bias=None):
@@ -102,7 +111,7 @@ def _layer_call(x, w, w_scale, w_add, out, ws, block, bias=None):
     (m, k), n, dev = x.shape, w.size(0), x.get_device()
     if (m == 0 or n == 0 or k == 0 or k > 65536 or w.size(1) * 2 != k or (k % block if block else k % 32)
             or x.dtype is not torch.bfloat16 or w.dtype is not torch.uint8 or w_scale.dtype is not torch.bfloat16
-            or w_add.dtype is not torch.int32 or w_scale.numel() != n or w_add.numel() != n
+            or w_add.dtype is not torch.int32 or w_scale.numel() < n or w_add.numel() < n
             or w.get_device() != dev or w_scale.get_device() != dev or w_add.get_device() != dev
             or not (x.is_contiguous() and w.is_contiguous() and w_scale.is_contiguous() and w_add.is_contiguous())):
         return None
@@ -127,7 +136,7 @@ def _layer_call(x, w, w_scale, w_add, out, ws, block, bias=None):
     else:
         a, a_scale, a_sums = ws
         if (a.shape not in ((m, k), (m, k // 2)) or a.dtype is not torch.uint8 or a_scale.dtype is not torch.bfloat16
-                or a_sums.dtype is not torch.int32 or a_scale.numel() != m or a_sums.numel() != m
+                or a_sums.dtype is not torch.int32 or a_scale.numel() < m or a_sums.numel() < m
                 or a.get_device() != dev or a_scale.get_device() != dev or a_sums.get_device() != dev
                 or not (a.is_contiguous() and a_scale.is_contiguous() and a_sums.is_contiguous()) or a.data_ptr() % 16):
             return None
@@ -177,45 +186,26 @@ def linear_forward(
 
     Where the library finds it faster the quantiser writes the GEMM's int8 operand directly (``_a_int8`` [M, K] uint8 is its
     workspace) instead of packed int4: same codes, same result, no unpack of A inside the GEMM.  A caller that passes
-    ``_a_int_packed`` but no ``_a_int8`` keeps the packed route.
+    ``_a_int_packed`` but no ``_a_int8`` keeps the packed route; of both, the one of the library's choice is written.
 
     With dense buffers the layer is ONE library call (``_layer_call``): the quantiser (with or without the transform, each
     row read once), then the GEMM kernel, where it pays launched with a programmatic dependency on the quantiser so that
     its set-up and first weight copies overlap the quantiser's end."""
     if w_meta_e is not None:
         raise NotImplementedError("quest_b200 implements the dense W4A4 path only")
-    if not debug_mode and (not use_hadamard or block in _BLOCKS):
-        codes = _a_int_packed if _a_int8 is None else _a_int8
-        if _a_int8 is not None and _a_int_packed is not None and not quest.prefers_a8(*activation.shape, w_int_packed.size(0)):
-            codes = _a_int_packed
-        ws = None
-        if codes is not None and _a_scale is not None and _a_int_row_sum is not None:
-            ws = (codes, _a_scale, _a_int_row_sum)
-        if ws is not None or (codes is None and _a_scale is None and _a_int_row_sum is None):
-            y = _layer_call(activation, w_int_packed, w_scale, w_add, out, ws, block if use_hadamard else 0)
-            if y is not None:
-                return y
+    if not debug_mode and activation.dim() == 2 and (not use_hadamard or block in _BLOCKS):
+        ws = _caller_workspaces(activation, w_int_packed.size(0), _a_int8, _a_int_packed, _a_scale, _a_int_row_sum)
+        y = _layer_call(activation, w_int_packed, w_scale, w_add, out, ws, block if use_hadamard else 0)
+        if y is not None:
+            return y
     M, K, N = activation.size(0), activation.size(1), w_int_packed.size(0)
     dtype, device = activation.dtype, activation.device
     if out is None:
         out = torch.empty(M, N, dtype=dtype, device=device)
     a_scale = torch.empty(M, 1, dtype=dtype, device=device) if _a_scale is None else _a_scale
     a_int_row_sum = torch.empty(M, 1, dtype=torch.int32, device=device) if _a_int_row_sum is None else _a_int_row_sum
-    if (use_hadamard and not debug_mode and (_a_int8 is not None or _a_int_packed is None) and K % block == 0
-            and quest.prefers_a8(M, K, N)):
-        a_int8 = torch.empty(M, K, dtype=torch.uint8, device=device) if _a_int8 is None else _a_int8
-        if _one_call_ok(activation, out, a_int8, a_scale, a_int_row_sum, w_int_packed, w_add, w_scale):
-            return quest.w4a4_linear_hadamard(activation, w_int_packed, w_add, w_scale, out, a_int8, a_scale, a_int_row_sum,
-                                              block=block)
-        quest.hadamard_quantize_a8(activation, block=block, x_a8=a_int8, scale=a_scale, x_int_row_sum=a_int_row_sum)
-        quest.fused_matmul_dequantize_a8(mat_a8=a_int8, mat_b=w_int_packed, vec_a_add=a_int_row_sum, vec_b_add=w_add,
-                                         vec_a_mul=a_scale, vec_b_mul=w_scale, out=out)
-        return out
     a_int_packed = torch.empty(M, K // 2, dtype=torch.uint8, device=device) if _a_int_packed is None else _a_int_packed
-    if use_hadamard and not debug_mode and _one_call_ok(activation, out, a_int_packed, a_scale, a_int_row_sum, w_int_packed, w_add, w_scale):
-        # one library call: the GEMM kernel starts behind the quantiser with a dependent launch
-        return quest.w4a4_linear_hadamard(activation, w_int_packed, w_add, w_scale, out, a_int_packed, a_scale, a_int_row_sum,
-                                          block=block)
+    assert w_int_packed.size(1) * 2 == K and (debug_mode or not use_hadamard or out.shape == (M, N))
     if use_hadamard:
         quest.hadamard_quantize_int4(activation, block=block, x_int_packed=a_int_packed, scale=a_scale,
                                      x_int_row_sum=a_int_row_sum)

@@ -95,3 +95,13 @@ def test_product_does_not_import_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h")):
                 text = open(os.path.join(dirpath, f)).read()
                 assert "oracle" not in text, os.path.join(dirpath, f)
+
+
+def test_linear_forward_refuses_a_batch_of_matrices():
+    """With both code buffers given, too (the choice between them asks for M, K and N)."""
+    import quest_b200 as quest
+    x = torch.zeros(2, 3, 128, dtype=torch.bfloat16)
+    codes = {"_a_int8": torch.zeros(2, 128, dtype=torch.uint8), "_a_int_packed": torch.zeros(2, 64, dtype=torch.uint8)}
+    with pytest.raises(AssertionError):
+        quest.linear_forward(x, torch.zeros(4, 64, dtype=torch.uint8), torch.zeros(4, 1, dtype=torch.bfloat16),
+                             torch.zeros(4, 1, dtype=torch.int32), use_hadamard=True, **codes)
