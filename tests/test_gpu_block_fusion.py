@@ -91,16 +91,27 @@ def test_rmsnorm_kernel(m, k):
 
 
 def test_silu_quotient_keeps_every_rounding():
-    """The gate of the fused quantiser against torch's silu over all bf16 values: the block is quantised with a scale that
-    the gate itself decides, so every value is put alone into a row of its own next to a fixed one."""
-    bits = torch.arange(65536, device=DEV, dtype=torch.int32).to(torch.int16)
-    vals = bits.view(torch.bfloat16)
-    vals = vals[vals.isfinite()]
-    gate = torch.zeros(vals.numel(), 64, dtype=torch.bfloat16, device=DEV)
-    gate[:, 0] = vals
-    up = torch.ones_like(gate)
-    ref = quest.hadamard_quantize_int4(torch.nn.functional.silu(gate) * up, 64)
-    got = quest.silu_mul_hadamard_quantize_int4(gate, up, 64)
-    ok = torch.isfinite(ref[1].flatten())
-    # the row's scale is a function of silu(v) alone, monotone in its magnitude: a gate rounded the other way moves it
-    assert got[1].flatten()[ok].equal(ref[1].flatten()[ok])
+    """The gate of the fused quantiser against torch's silu over all bf16 values.  Every value v sits alone in a row, next to a
+    factor that brings silu(v) near 1 (a power of two, exact), so that the row's scale is a rounded multiple of it; several
+    multiples of the factor, because one alone maps neighbouring values to one scale here and there."""
+    v = torch.arange(65536, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    v = v[v.isfinite()]
+    s = torch.nn.functional.silu(v)
+    near_one = torch.exp2((1 - torch.frexp(s.double())[1].double()).clamp(-126, 126))  # v below -88 gives -0: any factor
+
+    def row(first, rest=0.0):
+        t = torch.full((v.numel(), 64), rest, dtype=torch.bfloat16, device=DEV)
+        t[:, 0] = first
+        return t
+
+    seen = {-1: torch.zeros_like(v, dtype=torch.bool), 1: torch.zeros_like(v, dtype=torch.bool)}
+    for multiple in (1.0, 1.1875, 1.375, 1.5, 1.6875, 1.875):
+        up = row((near_one * multiple).to(torch.bfloat16), 1.0)
+        ref = quest.hadamard_quantize_int4(row(s) * up, 64)
+        got = quest.silu_mul_hadamard_quantize_int4(row(v), up, 64)
+        assert all(a.equal(b) for a, b in zip(got, ref)), multiple  # codes (the sign), scales, row sums
+        for step in seen:  # the same row with the value one unit in the last place off
+            other = (s.view(torch.int16) + step).view(torch.bfloat16)
+            seen[step] |= (quest.hadamard_quantize_int4(row(other) * up, 64)[1] != ref[1]).flatten()
+    nonzero = s != 0
+    assert seen[-1][nonzero].all() and seen[1][nonzero].all()  # ... shows, so the comparison above can fail
