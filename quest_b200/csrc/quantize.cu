@@ -858,8 +858,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict_
     for (int row = blockIdx.x * 8 + (threadIdx.x >> 5); row < M; row += gridDim.x * 8) {
         const __nv_bfloat16* xr = x + (size_t)row * K;
         uint4 held[8];
-        float sum = 0.f;
+        double total = 0.0;  // of pieces summed in eight chains of eight: a longer fp32 chain loses bits from K = 4096 on
         for (int base = 0; base < K; base += 2048) {
+            float part[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int e = base + (j * 32 + lane) * 8;
@@ -868,14 +869,16 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(__nv_bfloat16* __restrict_
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const uint32_t v[4] = {held[j].x, held[j].y, held[j].z, held[j].w};
+                part[j] = 0.f;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float a = bf16lo_to_f32(v[i]), b = bf16hi_to_f32(v[i]);
-                    sum = fmaf(a, a, sum);
-                    sum = fmaf(b, b, sum);
+                    part[j] = fmaf(b, b, fmaf(a, a, part[j]));
                 }
             }
+            total += (double)(((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7])));
         }
+        float sum = (float)total;
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
         const float rinv = rsqrtf(__fdiv_rn(sum, (float)K) + eps);

@@ -90,6 +90,18 @@ def test_rmsnorm_kernel(m, k):
     assert (y.double() - exact).abs().le(2 * 2.0 ** -8 * exact.abs() * 1.01 + 1e-30).all()
 
 
+@pytest.mark.parametrize("c", [1.0078125, 1.4140625, 1.8046875])
+@pytest.mark.parametrize("k", [2048, 65536])
+def test_rmsnorm_sums_long_rows(c, k):
+    """A constant row whose squares one long fp32 chain rounds down: at 2048 terms per lane (K = 65536) such a sum is 1.5e-5 to
+    3e-5 low and c * rinv half of that high.  eps puts the exact quotient 0.35e-5 below the tie between the two largest bf16
+    values up to 1, a margin of fifty fp32 roundings."""
+    tie = 1 - 2.0 ** -9
+    t = tie * (1 - 0.35e-5)
+    y = quest.rmsnorm(torch.full((3, k), c, dtype=torch.bfloat16, device=DEV), torch.ones(k, dtype=torch.bfloat16, device=DEV), c * c * (t ** -2 - 1))
+    assert (y == 1 - 2.0 ** -8).all()
+
+
 def test_silu_quotient_keeps_every_rounding():
     """The gate of the fused quantiser against torch's silu over all bf16 values.  Every value v sits alone in a row, next to a
     factor that brings silu(v) near 1 (a power of two, exact), so that the row's scale is a rounded multiple of it; several
