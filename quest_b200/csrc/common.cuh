@@ -75,6 +75,8 @@ extern thread_local bool qb_tl_in_layer;
 // Which kernel the last hadamard_quantize_int4_cuda_bf16 call of this host thread launched (the one-call layer decides
 // by it how to launch its GEMM).
 constexpr int kQuantiserTc = 1, kQuantiserMma = 2;
+// Elements from which a layer's quantiser is the tcgen05 kernel (see the crossover at hadamard_quantize_int4_cuda_bf16).
+constexpr long long kTcFromInLayer = 3ll * 1024 * 1024;
 extern thread_local int qb_tl_quantiser_kernel;
 
 // Reads and clears the device status word of the row-kernel translation unit (see tcgen05.cuh).

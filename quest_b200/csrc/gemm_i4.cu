@@ -1664,9 +1664,10 @@ using namespace qb;
 //    GEMM is launched behind it: -1 ... -2 us per layer;
 //  * below that the quantiser is the small CUDA-core kernel in plain stream order and only the GEMM is dependent (its
 //    set-up and first weight requests overlap the quantiser): -1.5 us per layer at M = 64 ... 512, K = 4096;
-//  * behind the CUDA-core quantiser of a large input the GEMM may be scheduled when the quantiser's blocks have done
-//    their last rows, not when they start: its waiting blocks would take their place (+1 ... +10 us at 4 M elements and
-//    more).
+//  * behind the CUDA-core quantiser of a large input only a GEMM on the int8 operand is dependent, scheduled when the
+//    quantiser's blocks have done their last rows (M 1000 K 11008 N 4096: 49.2 -> 47.2 us); a packed GEMM launched that way
+//    is slower (M 8192 K 11008 N 1024 152.6 against 140.6 us, M 2048 N 4096 96.6 against 84.3, M 14127 K 7296 N 1344
+//    199.5 against 194.9), because all its threads wait and its blocks hold the quantiser's place meanwhile.
 // QB200_DEPENDENT_LAUNCH in the environment (tests, tuning) forces the launches instead: bit 0 = the GEMM, bit 1 = the
 // quantiser is launched with a programmatic dependency; 0 = both in plain stream order.
 static thread_local bool tl_layer_mode = false;
@@ -1677,10 +1678,11 @@ static int dependent_launch_mask() {
 }
 
 // Before a GEMM launch: inside a layer the kernel before it in the stream is the layer's quantiser.
-static void note_layer_launch() {
+static void note_layer_launch(bool int8_operand, int M, int K) {
     if (!tl_layer_mode) return;
     const int mask = dependent_launch_mask();
-    tl_dependent_launch = mask >= 0 ? (mask & 1) != 0 : qb_tl_quantiser_kernel != 0;
+    const bool behind_mma = qb_tl_quantiser_kernel == kQuantiserMma && (int8_operand || (long long)M * K < kTcFromInLayer);
+    tl_dependent_launch = mask >= 0 ? (mask & 1) != 0 : (qb_tl_quantiser_kernel == kQuantiserTc || behind_mma);
     qb_tl_quantiser_kernel = 0;  // consumed: a second GEMM of the layer follows a GEMM, not the quantiser
 }
 
@@ -1691,7 +1693,7 @@ static int run_gemm_a8(const EpilogueParams& ep_in, const void* mat_a8, const vo
     int dev = 0;
     const int sms = sm_count_of_current_device(&dev);
     if (sms < 2) return QB200_ERR_CUDA;
-    note_layer_launch();
+    note_layer_launch(true, M, K);
     const int st = launch_gemm_a8(ep, mat_a8, mat_b, M, K, N, sms, dev, stream);
     tl_dependent_launch = false;
     return st;
@@ -1699,7 +1701,7 @@ static int run_gemm_a8(const EpilogueParams& ep_in, const void* mat_a8, const vo
 
 static int run_gemm(bool fused, const EpilogueParams& ep, const void* a, const void* b, int M, int K, int N,
                     cudaStream_t stream, int static_splits = -1) {
-    note_layer_launch();
+    note_layer_launch(false, M, K);
     const int st = run_gemm_impl(fused, ep, a, b, M, K, N, stream, static_splits);
     tl_dependent_launch = false;
     return st;

@@ -21,8 +21,6 @@ thread_local bool qb_tl_dependent_quantiser = false;
 thread_local bool qb_tl_in_layer = false;
 thread_local int qb_tl_quantiser_kernel = 0;
 
-constexpr long long kTcFromInLayer = 3ll * 1024 * 1024;  // elements; see the crossover at hadamard_quantize_int4_cuda_bf16
-
 struct RowParams {
     const __nv_bfloat16* x;        // [M,K] input
     __nv_bfloat16* x_out;          // optional [M,K] output (transformed or dequantised values)
