@@ -1800,10 +1800,12 @@ extern "C" int quest_b200_layer_operand(int M, int K, int N) {
     int dev = 0;
     const int sms = sm_count_of_current_device(&dev);
     if (sms < 2) return 0;
-    // For a few rows the dp4a kernel on packed codes streams the weights faster (layer, packed / int8, M 2: K 8192 N 10240
-    // 13.0 / 15.5 us; M 4: K 8192 N 3584 9.7 / 12.3; M 3: K 8192 N 10240 17.1 / 15.5, K 11008 N 4096 12.5 / 11.5), except
-    // for a long K with few weight rows, which leave it too few warps (M 1 K 28672 N 1024: 20.4 / 14.8).
-    if (gemv_eligible(M, K, N, 0) && (M <= 2 || (M <= 4 && (long long)M * N * K <= 120000000ll)) && !(K > 16384 && N < 4096)) return 0;
+    // For a few rows the dp4a kernel on packed codes streams the weights faster.  Per layer, weights from HBM, packed / int8:
+    // M 2 K 8192 N 10240 14.0 / 25.3 us, M 4 K 1408 N 9464 7.6 / 8.4; of three and four rows only up to 120 M multiply-adds
+    // (M 4 K 8192 N 3584 10.8 / 11.2, K 11008 N 4096 14.2 / 12.8) or with 8192 weight rows and more, where the few-token
+    // kernel needs several rounds (M 3 K 4096 N 11008 12.3 / 14.2, K 6400 N 9748 16.9 / 19.1, K 8192 N 10240 18.2 / 25.5);
+    // never with a long K and few weight rows, which leave it too few warps (M 1 K 28672 N 1024: 20.4 / 14.8).
+    if (gemv_eligible(M, K, N, 0) && (M <= 2 || (M <= 4 && ((long long)M * N * K <= 120000000ll || N >= 8192))) && !(K > 16384 && N < 4096)) return 0;
     // A narrow layer on a large input pays for the operand's second byte: M 7008 K 28672 N 1024 261 against 271 us.
     return (long long)M * K <= (48ll << 20) || N >= 1536;
 }
