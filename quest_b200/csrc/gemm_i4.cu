@@ -1441,8 +1441,10 @@ static long long pair_cycles(int M, int K, int N, int sms) {
 // kernel elsewhere.  QB200_A8_KERNEL=pair|skinny forces one (tests, tuning).
 static int launch_gemm_a8(const EpilogueParams& ep, const void* a8, const void* b, int M, int K, int N, int sms, int dev,
                           cudaStream_t stream) {
-    // Up to 32 rows the skinny kernel whatever the estimates say: seven eighths of a pair's rows would be empty.
-    bool use_skinny = M <= 32 || (M <= 128 && pick_skinny(skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms));
+    // Up to 32 rows the skinny kernel whatever the estimates say: seven eighths of a pair's rows would be empty.  Up to 128 rows
+    // also where output rows are not made of 16-byte pieces: a thread of the pair kernel then stores its own row two bytes at
+    // a time (M 122 K 1408 N 8513: 26.0 against 11.7 us), a warp of the skinny kernel 128 neighbouring columns.
+    bool use_skinny = M <= 32 || (M <= 128 && (ep.vec_ok == 0 || pick_skinny(skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms)));
     if (const char* e = getenv("QB200_A8_KERNEL")) use_skinny = e[0] == 's' && M <= 128;
     if (!use_skinny) return launch_gemm_pair(ep, a8, b, M, K, N, sms, dev, stream);
     switch (skinny_tokens(M)) {
