@@ -1884,10 +1884,10 @@ extern "C" int scale_quantize_int4_cuda_bf16(void*, void*, void*, const void*, i
 
 // How a layer that is free to choose runs: 0 packed codes, 1 int8 operand, 2 one kernel (no workspace at all).
 extern "C" int quest_b200_layer_plan(int M, int K, int N, int block) {
-    int per;
-    if (M > 0 && N > 0 && K > 0 && getenv("QB200_GEMM_TILE") == nullptr && getenv("QB200_GEMM_SPLITS") == nullptr &&
+    int per, dev = 0;
+    if (M > 0 && M <= 4 && N > 0 && K > 0 && getenv("QB200_GEMM_TILE") == nullptr && getenv("QB200_GEMM_SPLITS") == nullptr &&
         getenv("QB200_GEMM_GEMV") == nullptr && getenv("QB200_A8") == nullptr && getenv("QB200_HQ_KERNEL") == nullptr &&
-        gemv_layer_parts(M, K, N, block, &per) > 0)
+        gemv_layer_parts(M, K, N, block, sm_count_of_current_device(&dev), &per) > 0)
         return 2;
     return quest_b200_layer_operand(M, K, N);
 }

@@ -261,13 +261,17 @@ static int run_gemv(const EpilogueParams& ep, const void* a, const void* b, int 
 }
 
 // Rows that one block can quantise with a warp per row part (W parts of `per` units, as hadamard_quant_mma_kernel deals
-// them out), behind the Hadamard transform, where that measured no slower than two kernels (layer, launches back to back):
-// M 1 / 2 / 4 at K = N = 4096 6.0 / 6.2 / 7.5 -> 5.2 / 5.9 / 7.3 us, M 1 K 8192 N 10240 equal; beyond 100 M
-// multiply-adds the streaming of the weights is what counts and the plain kernel's four blocks per SM win (M 1 K 8192
-// N 28672 22.3 against 27.7 us).
-static int gemv_layer_parts(int M, int K, int N, int block, int* per_out) {
+// them out), behind the Hadamard transform, while two blocks per SM hold all weight rows at once.  Per layer, weights from
+// HBM, two kernels / one: M 1 K 4096 N 4096 7.7 / 6.6 us, M 4 8.2 / 8.2, M 1 K 2048 N 5632 6.1 / 5.6, M 2 K 8192 N 3584
+// 10.7 / 10.3.  Near the end of the range it takes up to a microsecond more (M 2 K 4096 N 8192 8.7 / 9.5) and saves the
+// caller a launch and an allocation (a call 16.5 / 11.2).  In a second round of blocks most SMs would idle, and every block
+// repeats the rows (M 1 K 4096 N 11008 9.2 / 11.5, K 8192 N 10240 12.9 / 17.0; with three blocks per SM 10.2 and 14.2).
+// Beyond 100 M multiply-adds the plain kernel's four blocks per SM stream the weights faster.
+constexpr int kLayerBlocksPerSm = 2, kLayerC = 4;
+static int gemv_layer_parts(int M, int K, int N, int block, int sms, int* per_out) {
     if (M < 1 || M > 4 || (block != 64 && block != 128 && block != 256) || K % block != 0) return 0;
     if (!gemv_eligible(M, K, N, 0) || (long long)M * N * K > 100000000ll) return 0;
+    if ((long long)N > (long long)kLayerC * gemv::kWarps * kLayerBlocksPerSm * sms) return 0;
     const int units = (K + kUnit - 1) / kUnit;
     const int per = units >= 2 ? 2 : 1;
     const int W = (units + per - 1) / per;
@@ -278,7 +282,7 @@ static int gemv_layer_parts(int M, int K, int N, int block, int* per_out) {
 template <int MR, int HB, int UNITS>
 static int launch_gemv_layer(const EpilogueParams& ep, const void* x, const void* b, int M, int K, int N, int W, int sms, int dev,
                              cudaStream_t stream) {
-    constexpr int C = 4;
+    constexpr int C = kLayerC;
     static bool attr_set[64] = {false};
     auto kernel = gemv_layer_kernel<MR, C, HB, UNITS>;
     const size_t smem = (size_t)MR * (size_t)(K / 2) + (size_t)gemv::kWarps * UNITS * kStepIn;
@@ -289,9 +293,7 @@ static int launch_gemv_layer(const EpilogueParams& ep, const void* x, const void
         }
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    int grid = ((N + C - 1) / C + gemv::kWarps - 1) / gemv::kWarps;
-    const int per_sm = smem > 100 * 1024 ? 1 : 2;
-    if (grid > sms * per_sm) grid = sms * per_sm;
+    const int grid = ((N + C - 1) / C + gemv::kWarps - 1) / gemv::kWarps;  // all resident, see gemv_layer_parts
     const float had_scale = __bfloat162float(__float2bfloat16_rn((float)(1.0 / sqrt((double)HB))));
     kernel<<<grid, gemv::kThreads, smem, stream>>>(static_cast<const __nv_bfloat16*>(x), static_cast<const uint8_t*>(b), ep, M, N, K, W, had_scale);
     return launch_status();
@@ -301,7 +303,7 @@ template <int MR, int HB>
 static int launch_gemv_layer_units(const EpilogueParams& ep, const void* x, const void* b, int M, int K, int N, int sms, int dev,
                                    cudaStream_t stream) {
     int per = 0;
-    const int W = gemv_layer_parts(M, K, N, HB, &per);
+    const int W = gemv_layer_parts(M, K, N, HB, sms, &per);
     if (W == 0) return QB200_ERR_UNSUPPORTED;
     if (per == 1) return launch_gemv_layer<MR, HB, 1>(ep, x, b, M, K, N, W, sms, dev, stream);
     return launch_gemv_layer<MR, HB, 2>(ep, x, b, M, K, N, W, sms, dev, stream);

@@ -29,6 +29,20 @@ def test_one_kernel_layer_equals_quantiser_and_gemm(m, k, one_kernel, block):
     assert quest.linear_forward(zero, wp, ws, wa, use_hadamard=True, block=block).isfinite().all()
 
 
+# as many weight rows as two blocks per SM hold, and one more
+@pytest.mark.parametrize("m", [1, 2])
+def test_one_kernel_layer_runs_in_one_round(m):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for n, one_kernel in ((64 * sms, True), (64 * sms + 1, False)):
+        g = torch.Generator(device=DEV).manual_seed(n)
+        w = (0.02 * torch.randn(n, 1024, device=DEV, generator=g)).to(torch.bfloat16)
+        wp, ws, wa, _ = quest.preprocess_weight(w, use_hadamard=True)
+        x = torch.randn(m, 1024, device=DEV, generator=g).to(torch.bfloat16)
+        assert (_lib.load().quest_b200_layer_plan(m, 1024, n, 128) == 2) == one_kernel
+        packed, scale, sums = quest.hadamard_quantize_int4(x)
+        assert quest.linear_forward(x, wp, ws, wa, use_hadamard=True).equal(quest.fused_matmul_dequantize_int4_int4t_bf16(packed, wp, sums, wa, scale, ws))
+
+
 @pytest.mark.parametrize("use_hadamard", [True, False])
 @pytest.mark.parametrize("m,k,n", [(1, 2048, 96), (12, 2048, 200), (100, 2048, 264), (333, 2048, 1001), (20, 96, 40)])
 def test_module_bias(m, k, n, use_hadamard):
