@@ -1366,26 +1366,38 @@ struct SkinnyPlan {
     long long cycles;  // estimated
 };
 
-// Weight rows per CTA and K ranges of the skinny kernel, in cycles.  Measured (K = 4096, N = 11008 and 12288): a step of
-// 128 K takes 440 / 475 / 565 / 720 cycles of an SM at 16 / 32 / 64 / 128 tokens whatever the weight rows are (the issue
-// of four MMAs, then the tokens' way through shared memory), a launch about 8000 cycles, the exchange of a cluster 2500
-// and each wave of CTAs beyond the first about 3000.  Larger clusters do not reach every SM: with one CTA per SM, clusters
-// of four and eight leave 16 and 28 of 148 SMs without one (the occupancy calculator's count; with splits of three and
-// more estimated on 144 SMs, M 81 K 2048 N 6144 took 18.6 instead of 13.3 us).
-static SkinnyPlan pick_skinny(int tn, int K, int N, int sms) {
+// Weight rows per CTA and K ranges of the skinny kernel, in cycles; the constants fit 10 shapes x 6 row counts x 7 plans (device
+// time of the layer, weights from HBM) within 8 %.  A step of 128 K takes a CTA that has the SM for itself 430 / 430 / 425 / 475
+// cycles at 16 / 32 / 64 / 128 tokens whatever its weight rows are (the issue of four MMAs, then the tokens' way through shared
+// memory); two CTAs on one SM (up to 32 tokens) take 280 + 3.5 per weight row for a step of each.  Every wave of CTAs costs its
+// start, fill and epilogue again: 11000 to 14500 cycles.  The exchange of a cluster of S costs about 500 S.
+// Larger clusters do not reach every SM: with one CTA per SM, clusters of four and eight leave 16 and 28 of 148 SMs without one
+// (the occupancy calculator's count).  Up to 32 tokens the CTAs are scheduled while the quantiser still holds a place on an SM
+// per row: clusters of four and eight beyond the free places wait for a second wave (K 28672 N 8192 at 16 rows: 276 CTAs
+// 50.3 us, 256 CTAs 32.7), and where fewer SMs are free than there are CTAs some SMs get two (128 CTAs at 20 / 24 rows: 41.6 /
+// 58.1), which fewer weight rows per CTA do not mend.
+// Device time at 16 and 32 rows, the plan of one cost per step and 3000 per wave -> this one's: K 4096 N 22016 26.1, 27.9 ->
+// 17.0, 18.3 us; K 8192 N 10240 26.9, 28.7 -> 17.6, 18.7; K 28672 N 8192 41.0, 58.5 -> 32.7, 35.9.
+static SkinnyPlan pick_skinny(int M, int tn, int K, int N, int sms) {
     const int num_kb = K / BK;
-    const int per_sm = tn <= 32 ? 2 : 1;
-    const long long step = tn <= 16 ? 440 : (tn <= 32 ? 475 : (tn <= 64 ? 565 : 720));
+    const bool share = tn <= 32;
+    const int step = tn <= 32 ? 430 : (tn <= 64 ? 425 : 475), wave = tn <= 32 ? 11000 : (tn <= 64 ? 12000 : 14500);
     SkinnyPlan best{0, 0, -1};
     for (int s = 1; s <= skinny::kMaxSplit && s <= num_kb; s *= 2) {
         int usable = sms;
-        if (s > 2) usable = per_sm == 2 ? sms - 4 : (s == 4 ? sms - 16 : sms - 28);
+        if (s > 2) usable = share ? sms - 4 : (s == 4 ? sms - 16 : sms - 28);
         if (usable < s) continue;
-        for (int rows = skinny::W_ROWS; rows >= 8; rows -= 8) {
+        const int kb = (num_kb + s - 1) / s;
+        for (int rows = skinny::W_ROWS; rows >= 64; rows -= 8) {  // fewer rows do not shorten a step
             const long long ctas = (long long)((N + rows - 1) / rows) * s;
-            const long long waves = (ctas + (long long)usable * per_sm - 1) / ((long long)usable * per_sm);
-            const long long steps = (ctas + usable - 1) / usable * ((num_kb + s - 1) / s);  // of the busiest SM
-            const long long t = steps * step + 8000 + (waves - 1) * 3000 + (s > 1 ? 2500 : 0) + tn * 10;
+            long long places = share ? 2 * usable : usable;
+            if (share && s > 2) places = places > M ? places - M : 1;
+            const long long waves = (ctas + places - 1) / places, per_sm = (ctas + usable - 1) / usable;  // of the busiest SM
+            long long steps = per_sm * step;
+            if (share && per_sm > 1) steps = per_sm / 2 * (280 + rows * 7 / 2) + per_sm % 2 * step;
+            else if (share && ctas > usable - M) steps = 280 + skinny::W_ROWS * 7 / 2;
+            // ... and the start of a second CTA, and the exchange
+            const long long t = steps * kb + waves * wave + (share && per_sm > 1 ? 2000 : 0) + (s > 1 ? 500 * s : 0);
             if (best.cycles < 0 || t < best.cycles) best = SkinnyPlan{rows, s, t};
         }
     }
@@ -1407,7 +1419,7 @@ static int launch_gemm_skinny_tn(const EpilogueParams& ep, const void* a8, const
             return QB200_ERR_CUDA;
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    const SkinnyPlan plan = pick_skinny(TN, K, N, sms);
+    const SkinnyPlan plan = pick_skinny(M, TN, K, N, sms);
     CUtensorMap mw, mt;
     int st = make_packed_map(&mw, b, N, K, plan.rows);
     if (st != QB200_OK) return st;
@@ -1441,10 +1453,11 @@ static long long pair_cycles(int M, int K, int N, int sms) {
 // kernel elsewhere.  QB200_A8_KERNEL=pair|skinny forces one (tests, tuning).
 static int launch_gemm_a8(const EpilogueParams& ep, const void* a8, const void* b, int M, int K, int N, int sms, int dev,
                           cudaStream_t stream) {
-    // Up to 32 rows the skinny kernel whatever the estimates say: seven eighths of a pair's rows would be empty.  Up to 128 rows
+    // Up to 32 rows the skinny kernel whatever the estimates say: seven eighths of a pair's rows would be empty (M 32, pair /
+    // skinny: K 28672 N 8192 62.4 / 36.0 us, K 8192 N 28672 44.6 / 35.8, K 4096 N 12288 17.6 / 15.5).  Up to 128 rows
     // also where output rows are not made of 16-byte pieces: a thread of the pair kernel then stores its own row two bytes at
     // a time (M 122 K 1408 N 8513: 26.0 against 11.7 us), a warp of the skinny kernel 128 neighbouring columns.
-    bool use_skinny = M <= 32 || (M <= 128 && (ep.vec_ok == 0 || pick_skinny(skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms)));
+    bool use_skinny = M <= 32 || (M <= 128 && (ep.vec_ok == 0 || pick_skinny(M, skinny_tokens(M), K, N, sms).cycles < pair_cycles(M, K, N, sms)));
     if (const char* e = getenv("QB200_A8_KERNEL")) use_skinny = e[0] == 's' && M <= 128;
     if (!use_skinny) return launch_gemm_pair(ep, a8, b, M, K, N, sms, dev, stream);
     switch (skinny_tokens(M)) {
