@@ -15,7 +15,7 @@ from torch.autograd import forward_ad
 
 import quest_b200 as quest
 from . import _lib
-from .workspace import default_cache
+from .workspace import default_cache, layer_workspaces
 
 HADAMARD_BLOCK = 128  # the reference hard-codes block 128 (utils.py:17, 39, 90)
 
@@ -129,7 +129,13 @@ def _layer_call(x, w, w_scale, w_add, out, ws, block, bias=None):
             codes = sums = scale = None
         else:
             code_bytes = -(-(m * k if int8 else m * (k // 2)) // 256) * 256
-            buf = x.new_empty(code_bytes // 2 + 3 * m)  # bf16 elements: two bytes each
+            try:
+                buf = x.new_empty(code_bytes // 2 + 3 * m)  # bf16 elements: two bytes each
+            except torch.OutOfMemoryError:  # a layer fits where its packed form does
+                if not int8:
+                    raise
+                int8, code_bytes = 0, -(-(m * (k // 2)) // 256) * 256
+                buf = x.new_empty(code_bytes // 2 + 3 * m)
             codes = buf.data_ptr()
             sums = codes + code_bytes
             scale = sums + 4 * m
@@ -281,8 +287,8 @@ class Linear4bit(nn.Module):
             plan = _lib.load().quest_b200_layer_plan(m, k, self.out_features, block)
             ws, buffers = {}, None
             if plan != 2:
-                ws = self.workspaces.get(m, k, a.device, a.dtype, int8_operand=plan == 1)
-                buffers = (ws["_a_int8"] if plan == 1 else ws["_a_int_packed"], ws["_a_scale"], ws["_a_int_row_sum"])
+                ws = layer_workspaces(self.workspaces, m, k, a.device, a.dtype, plan == 1)
+                buffers = (ws["_a_int8"] if "_a_int8" in ws else ws["_a_int_packed"], ws["_a_scale"], ws["_a_int_row_sum"])
             y = _layer_call(a, self.w_int_packed, self.w_scale, self.w_add, None, buffers, block, self.bias)
             if y is not None:
                 return y if x.dim() == 2 else y.view(*x.shape[:-1], self.out_features)

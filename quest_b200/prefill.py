@@ -19,7 +19,7 @@ from torch.autograd import forward_ad
 
 import quest_b200 as quest
 from .layer import HADAMARD_BLOCK, Linear4bit
-from .workspace import default_cache
+from .workspace import default_cache, layer_workspaces
 
 FUSED_MODES = ("int4_fused",)  # modes in which the quantiser is fused into the producer of each linear's input
 
@@ -124,7 +124,7 @@ class Block(nn.Module):
         m, ffn = flat.size(0), self.mlp.w1.out_features
 
         def ws(k, n):  # codes (int8 operand or packed), scales and row sums for a linear with k inputs and n outputs
-            w = default_cache.get(m, k, x.device, x.dtype, int8_operand=k % HADAMARD_BLOCK == 0 and quest.layer_operand(m, k, n))
+            w = layer_workspaces(default_cache, m, k, x.device, x.dtype, k % HADAMARD_BLOCK == 0 and quest.layer_operand(m, k, n))
             return dict(codes=w["_a_int8"] if "_a_int8" in w else w["_a_int_packed"], scale=w["_a_scale"], x_int_row_sum=w["_a_int_row_sum"])
 
         att = self.attn

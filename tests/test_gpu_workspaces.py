@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import quest_b200 as quest
+from quest_b200.workspace import WorkspaceCache
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -64,3 +65,29 @@ def test_buffers_of_other_shapes_are_still_refused():
     with pytest.raises(AssertionError):
         quest.linear_forward(x, wp, ws, wa, use_hadamard=True, out=torch.empty(m, n + 8, dtype=torch.bfloat16, device=DEV))
     assert quest.linear_forward(x[:0], wp, ws, wa, use_hadamard=True).shape == (0, n)
+
+
+@pytest.mark.parametrize("module", [False, True])
+def test_a_layer_fits_where_its_packed_form_does(module):
+    """With room for the output and the packed codes only: the allocator's own limit stands in for a full device."""
+    m, k, n = 32768, 8192, 1536
+    x, wp, ws, wa = layer(m, k, n)
+    lin = quest.Linear4bit(k, n, bias=False, device=DEV, dtype=torch.bfloat16, use_hadamard=True)
+    lin.w_int_packed, lin.w_scale, lin.w_add = wp, ws, wa
+    lin.workspaces = WorkspaceCache()
+    call = (lambda: lin(x)) if module else (lambda: quest.linear_forward(x, wp, ws, wa, use_hadamard=True))
+    assert quest.layer_operand(m, k, n)
+    with torch.inference_mode():
+        ref = call()
+        lin.workspaces.clear()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        room = 2 * m * n + m * k // 2 + (64 << 20)  # less than half of the int8 operand's second half to spare
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / torch.cuda.get_device_properties(0).total_memory)
+        try:
+            y = call()
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+    # the packed route may quantise with another kernel, which may round a transform output the other way
+    assert (y.float() - ref.float()).norm() <= 1e-2 * ref.float().norm()
+    assert not module or {"_a_int_packed"} == {name for ws_ in lin.workspaces._sets.values() for name in ws_ if name.startswith("_a_int") and name != "_a_int_row_sum"}
