@@ -179,8 +179,9 @@ int fused_matmul_dequantize_int4_int4t_bf16_push_cuda(void* const* mat_d_list, i
  * row-major, and inside every group of 32 consecutive K positions the 16 even positions first, then the 16 odd
  * ones - so that the GEMM need not unpack A.  Only shapes the tcgen05 quantiser can tile (group_size a multiple of
  * 128, see quest_b200_prefers_a8); QB200_ERR_UNSUPPORTED otherwise.  fused_matmul_dequantize_a8_int4t_bf16_cuda is the
- * fused GEMM + epilogue taking that operand (mat_b stays packed int4; K a multiple of 128).  quest_b200_prefers_a8 returns 1 where this route is the faster one for an [M, K] x [N, K]^T layer (what
- * quest_b200.layer.linear_forward asks before choosing), else 0; QB200_A8=0|1 in the environment overrides it.
+ * fused GEMM + epilogue taking that operand (mat_b stays packed int4; K a multiple of 128).  quest_b200_prefers_a8 returns 1
+ * where these two calls are faster than the two on packed codes for an [M, K] x [N, K]^T layer, else 0 (for the layer in one call
+ * see quest_b200_layer_operand); QB200_A8=0|1 in the environment overrides it.
  */
 int hadamard_quantize_a8_cuda_bf16(void* a8_ptr, void* scale_ptr, void* x_int_row_sum_ptr, const void* x_ptr,
                                    int group_size, int batch_size, int block, cudaStream_t stream);
@@ -198,8 +199,8 @@ int quest_b200_layer_operand(int M, int K, int N);
 /*
  * The layer in one call with or without (block 0) the Hadamard transform, on packed codes ([M, K/2]; int8_operand 0), on the
  * int8 operand ([M, K]; 1), or as one kernel that needs no codes, scales and row sums (2; they may be NULL): what
- * quest_b200.layer.linear_forward calls.  quest_b200_layer_plan returns the fastest of the three for a shape.  bias (bf16 [N], may be NULL) is added to the
- * bf16 result as a separate add would, where quest_b200_layer_adds_bias returns 1 (QB200_ERR_UNSUPPORTED elsewhere).
+ * quest_b200.layer.linear_forward calls.  quest_b200_layer_plan returns the fastest of the three for a shape.  bias (bf16 [N],
+ * may be NULL) is added to the bf16 result as a separate add would, where quest_b200_layer_adds_bias returns 1 (QB200_ERR_UNSUPPORTED elsewhere).
  * QB200_ERR_UNSUPPORTED for a block other than 0, 64, 128 or 256, and for block 0 in the one-kernel form.
  */
 int w4a4_linear_layer_cuda(void* mat_d, const void* x, const void* w_int_packed, const void* w_add, const void* w_scale,

@@ -683,8 +683,6 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 // on their own, at the latest when the grid ends): enough to let the CTA go.
 __device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-// At most the newest bulk group of this thread may still be reading its shared-memory source.
-__device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 
 // One warp's share of a 256 x 256 tile: its 32 rows (tensor-memory lanes) x the columns [c_begin, c_end), in pieces of 64.
 // stage_base == 0: every thread stores its row's results itself (32-byte pieces).  stage_base != 0 (fused output, the
@@ -1786,26 +1784,6 @@ extern "C" int fused_matmul_dequantize_a8_int4t_bf16_cuda(void* mat_d, const voi
     return run_gemm_a8(ep, mat_a8, mat_b, M, K, N, stream);
 }
 
-constexpr bool kA8ByDefault = true;  // measured faster wherever the 256 x 256 kernel and the tcgen05 quantiser both apply (QB200_A8=0 switches it off)
-
-// 1 if, for this layer shape, the int8-operand route (hadamard_quantize_a8_cuda_bf16 + the GEMM above) is the faster one:
-// the 256 x 256 kernel would be chosen anyway and the quantiser's tcgen05 kernel can tile K.
-extern "C" int quest_b200_prefers_a8(int M, int K, int N) {
-    if (M <= 0 || K <= 0 || N <= 0 || K % 128 != 0 || K >= (1 << 17)) return 0;
-    if (getenv("QB200_GEMM_TILE") != nullptr || getenv("QB200_GEMM_SPLITS") != nullptr) return 0;
-    if (const char* e = getenv("QB200_A8")) return e[0] != '0';
-    if (!kA8ByDefault) return 0;
-    int dev = 0;
-    const int sms = sm_count_of_current_device(&dev);
-    long long est = 0;
-    if (sms <= 0 || pick_tile(M, N, K, sms, &est) != kWideTile) return 0;
-    // The int8 operand is twice the packed one.  Up to 32 MB (M = 8192, K = 4096) the route measured 1-5 % faster, at
-    // 64 MB the same, beyond that slower (M = 65536, K = 4096: 889 against 791 us): the operand no longer stays in L2
-    // between the CTAs that share its rows.
-    if ((long long)M * K > (48ll << 20)) return 0;
-    return hq_tc_shape_ok(K) ? 1 : 0;
-}
-
 // 1 if the layer (quantiser and GEMM in one) takes the int8 operand: every K that is a multiple of 128, except for the
 // few rows where the dp4a kernel on packed codes is the faster one.
 extern "C" int quest_b200_layer_operand(int M, int K, int N) {
@@ -1823,6 +1801,15 @@ extern "C" int quest_b200_layer_operand(int M, int K, int N) {
     if (gemv_eligible(M, K, N, 0) && (M <= 2 || (M <= 4 && ((long long)M * N * K <= 120000000ll || N >= 8192))) && !(K > 16384 && N < 4096)) return 0;
     // A narrow layer on a large input pays for the operand's second byte: M 7008 K 28672 N 1024 261 against 271 us.
     return (long long)M * K <= (48ll << 20) || N >= 1536;
+}
+
+// The same for the two separate ops: their int8 operand comes from the tcgen05 quantiser alone, which must tile K and is the
+// faster quantiser from a few million elements on.  Quantiser + GEMM as separate launches, packed / int8: M 1024 K 2048 N 6144
+// 19.8 / 22.0 us, M 768 K = N = 4096 26.1 / 22.2, M 2048 37.4 / 36.2, M 8192 127 / 98, M 65536 1078 / 842.
+extern "C" int quest_b200_prefers_a8(int M, int K, int N) {
+    if (!quest_b200_layer_operand(M, K, N)) return 0;
+    if (getenv("QB200_A8") != nullptr) return 1;
+    return (long long)M * K >= kTcFromInLayer && hq_tc_shape_ok(K) ? 1 : 0;
 }
 
 extern "C" int fused_matmul_dequantize_int4_int4t_bf16_noalloc_cuda(void* mat_d, const void* mat_a, const void* mat_b,

@@ -119,3 +119,10 @@ def test_layer_routes_agree(m, k, n, use_hadamard):
         with pytest.raises(AssertionError):
             quest.linear_forward(torch.cat([x, x], dim=1)[:, :k], wp, ws, wa, use_hadamard=use_hadamard)
     assert quest.device_status() == 0
+
+
+def test_preference_of_the_separate_ops():
+    """The layer's rule, for what the tcgen05 quantiser tiles and is the faster quantiser for."""
+    for m, k, n, prefers in ((1024, 2048, 6144, False), (16, 4096, 4096, False), (2048, 5632, 2048, False), (768, 4096, 4096, True),
+                             (16384, 4096, 4096, True), (65536, 4096, 1024, False)):
+        assert quest.prefers_a8(m, k, n) == prefers, (m, k, n)
