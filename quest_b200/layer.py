@@ -285,11 +285,12 @@ class Linear4bit(nn.Module):
             m, k = a.shape
             block = HADAMARD_BLOCK if self.use_hadamard else 0
             plan = _lib.load().quest_b200_layer_plan(m, k, self.out_features, block)
+            out = a.new_empty((m, self.out_features))  # before the workspaces, which have a smaller form where memory is short
             ws, buffers = {}, None
             if plan != 2:
                 ws = layer_workspaces(self.workspaces, m, k, a.device, a.dtype, plan == 1)
                 buffers = (ws["_a_int8"] if "_a_int8" in ws else ws["_a_int_packed"], ws["_a_scale"], ws["_a_int_row_sum"])
-            y = _layer_call(a, self.w_int_packed, self.w_scale, self.w_add, None, buffers, block, self.bias)
+            y = _layer_call(a, self.w_int_packed, self.w_scale, self.w_add, out, buffers, block, self.bias)
             if y is not None:
                 return y if x.dim() == 2 else y.view(*x.shape[:-1], self.out_features)
             y = linear_forward(activation=a, w_int_packed=self.w_int_packed, w_scale=self.w_scale, w_add=self.w_add,
