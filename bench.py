@@ -43,15 +43,21 @@ L2_BYTES = 126 << 20
 # shape; the file under profiles/ holds the capture's command and figures.  Only these shapes report `traffic`.
 NCU_TRAFFIC = {
     # (kernel, M, K, N or None, int8-operand route?)
-    ("gemm", 2048, 4096, 4096, True): (16.86e6 + 2.0 * 2048 * 4096, "profiles/gemm_i4_wide_kernel_fused_m2048_k4096_n4096.md (A8 column): 16.86 MB"
-                                       " read by the kernel; its 16.78 MB of output are still in L2 when it ends and are written back afterwards"),
-    ("gemm", 2048, 4096, 4096, False): (12.67e6 + 2.0 * 2048 * 4096, "profiles/gemm_i4_wide_kernel_fused_m2048_k4096_n4096.md (packed column): 12.67 MB"
+    ("gemm", 2048, 4096, 4096, True): (16.85e6 + 2.0 * 2048 * 4096, "profiles/gemm_i4_pair_kernel_fused_m2048_k4096_n4096.md: 16.85 MB read"
+                                       " by the kernel; its 16.78 MB of output are still in L2 when it ends and are written back afterwards"),
+    ("gemm", 2048, 4096, 4096, False): (12.67e6 + 2.0 * 2048 * 4096, "profiles/gemm_i4_wide_kernel_fused_m2048_k4096_n4096.md: 12.67 MB"
                                         " read by the kernel; its 16.78 MB of output are still in L2 when it ends and are written back afterwards"),
     ("hadamard_quantize", 2048, 4096, None, True): (16.82e6 + 2048 * 4096 + 6.0 * 2048, "profiles/hadamard_quant_kernels_headline_and_large.md (first"
                                                     " column): the input is read exactly once, the outputs are written back after the kernel"),
     ("hadamard_quantize", 2048, 4096, None, False): (16.81e6 + 2048 * 4096 / 2 + 6.0 * 2048, "profiles/hadamard_quant_kernels_headline_and_large.md"
                                                      " (second column): the input is read exactly once, the outputs are written back after the kernel"),
 }
+
+
+def layer_route(m, k, n, block=128):
+    """How linear_forward runs a layer of this shape when it is free to choose."""
+    from quest_b200 import _lib
+    return ("packed int4", "int8 operand", "one kernel")[_lib.load().quest_b200_layer_plan(m, k, n, block)]
 
 
 # ----------------------------------------------------------------------------------------------------
@@ -341,8 +347,8 @@ def run_b200(args):
             layer = ShardedLinear4bit((wp, ws, wa), n_total, rank, world, use_hadamard=True, block=args.block, exchange="nccl")
     flush = torch.zeros(L2_FLUSH_BYTES // 4, dtype=torch.int32, device=dev)
 
-    # One GPU: the layer takes the route linear_forward takes.  Where the library prefers it (256 x 256 GEMM kernel and a
-    # row length the tcgen05 quantiser tiles) the quantiser writes the GEMM's int8 operand instead of packed int4.
+    # One GPU: the quantiser writes the GEMM's int8 operand instead of packed int4 where the library prefers that for the two
+    # separate ops (a row length the tcgen05 quantiser tiles, enough elements for it); the timed layer uses the same buffers.
     use_a8 = world == 1 and args.block in (64, 128, 256) and k % args.block == 0 and quest.prefers_a8(m, k, n_local)
     a_scale = torch.empty(m, 1, dtype=torch.bfloat16, device=dev)
     a_packed = torch.empty(m, k if use_a8 else k // 2, dtype=torch.uint8, device=dev)
@@ -722,8 +728,10 @@ def run_b200(args):
             "warmup": max(args.warmup, 3), "ms_per_step": t_main * 1e3, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "int4 operands, int8 tcgen05 MMA, int32 accumulate, bf16 out",
             "data": "synthetic", "config": workload_config(args, world),
-            "roofline": {"kernel": "gemm_i4_wide_kernel / gemm_i4_kernel (TMA -> int4 unpack -> tcgen05 kind::i8, fused dequant epilogue;"
-                                   " 256x256 tiles at the default shape, last tile of a CTA stored with bulk tensor stores)", "bound": "tensor",
+            "roofline": {"kernel": (("gemm_i4_pair_kernel (up to 128 rows gemm_i4_skinny_kernel): A as int8 by TMA, int4 weights unpacked, tcgen05 kind::i8,"
+                                     " fused dequant epilogue; at the default shape 256-row x 256-column tiles on pairs of CTAs (cta_group::2)")
+                                    if use_a8 else "gemm_i4_wide_kernel / gemm_i4_kernel / gemv_i4_kernel (TMA -> int4 unpack of A and B -> tcgen05 kind::i8, fused dequant epilogue)"),
+                         "bound": "tensor",
                          "achieved": ops_gemm / t_gemm_roof / 1e12 if t_gemm_roof > 0 else None, "peak": int8_peak,
                          "unit": "TOPS", "frac": (ops_gemm / t_gemm_roof / 1e12) / int8_peak if t_gemm_roof > 0 else None,
                          "peak_source": f"2 x bf16_tflops ({peaks['bf16_tflops']}) of {peaks['source']}",
@@ -731,8 +739,8 @@ def run_b200(args):
                          "traffic_source": gemm_traffic[1] if gemm_traffic else None,
                          "us_per_launch": t_gemm_roof * 1e6,
                          "us_per_launch_isolated": t_gemm * 1e6 if t_gemm > 0 else None,
-                         "route": ("int8 operand: the quantiser writes 16 x code as int8 in the GEMM's operand order, the 256x256 kernel copies A"
-                                   " with TMA and unpacks only B (the library's default where both kernels apply; QB200_A8=0 for packed A)")
+                         "route": ("int8 operand: the quantiser writes 16 x code as int8 in the GEMM's operand order, the GEMM copies A"
+                                   " with TMA and unpacks only B (QB200_A8=0 for packed A)")
                          if use_a8 else "packed int4 A and B, both unpacked in the kernel",
                          "timing": b2b_note.format(n=n_gemm_sets, mb=n_gemm_sets * (a_packed.numel() + n_local * k / 2 + 2.0 * m * n_local) / 1e6)
                          if t_gemm_b2b else "events between the step's kernels",
@@ -863,17 +871,11 @@ def run_c4(args):
                    "gemm_plus_f1_us": (t_gemm + t_f1) * 1e6,
                    "aggregate_tops_gemm_plus_f1": 2.0 * m * n_total * k / (t_gemm + t_f1) / 1e12}
             if world == 1:
-                # the whole layer as linear_forward runs it on one GPU: the route the library prefers for the shape (int8
-                # operand with balanced tile columns where the 256-row kernel applies), one call, dependent launches
-                a8 = quest.prefers_a8(m, k, n_local)
-                codes = torch.empty(m, k if a8 else k // 2, dtype=torch.uint8, device=dev)
-                ws_kw = {"_a_int8": codes} if a8 else {"_a_int_packed": codes}
-                t_layer = timed(lambda: quest.linear_forward(x, wp, ws, wa, out=local, _a_scale=sc, _a_int_row_sum=rs,
-                                                             use_hadamard=True, block=args.block, **ws_kw))
+                # the whole layer as linear_forward runs it on one GPU: the library's route, one call, dependent launches
+                t_layer = timed(lambda: quest.linear_forward(x, wp, ws, wa, out=local, use_hadamard=True, block=args.block))
                 row["layer_us"] = t_layer * 1e6
-                row["layer_route"] = "int8 operand" if a8 else "packed int4"
+                row["layer_route"] = layer_route(m, k, n_local, args.block)
                 row["aggregate_tops_layer"] = 2.0 * m * n_total * k / t_layer / 1e12
-                del codes
             if world > 1:
                 delivered = {}
                 for exch in ("push", "nccl"):
@@ -978,14 +980,9 @@ def run_layers(args):
             t_kernel = do_bench_network(
                 lambda a_in, a_out: quest.linear_forward(a_in, wp, ws, wa, out=a_out, _a_scale=a_scale, _a_int_packed=a_packed,
                                                          _a_int_row_sum=a_rsum, use_hadamard=False), m, k, n, dtype, dev)
-            # with the Hadamard transform the layer takes the route the library prefers for the shape
-            a8 = quest.prefers_a8(m, k, n)
-            had_ws = {"_a_int8": torch.empty(m, k, dtype=torch.uint8, device=dev)} if a8 else {"_a_int_packed": a_packed}
-            t_had = do_bench_network(
-                lambda a_in, a_out: quest.linear_forward(a_in, wp, ws, wa, out=a_out, _a_scale=a_scale, _a_int_row_sum=a_rsum,
-                                                         use_hadamard=True, **had_ws), m, k, n, dtype, dev)
-            del had_ws
-            table.append({"N": n, "K": k, "M": m, "route": "int8 operand" if a8 else "packed int4", "bf16_us": t_base * 1e6, "int4_us": t_kernel * 1e6, "int4_hadamard_us": t_had * 1e6,
+            # with the Hadamard transform the layer takes the library's route for the shape
+            t_had = do_bench_network(lambda a_in, a_out: quest.linear_forward(a_in, wp, ws, wa, out=a_out, use_hadamard=True), m, k, n, dtype, dev)
+            table.append({"N": n, "K": k, "M": m, "route": layer_route(m, k, n), "bf16_us": t_base * 1e6, "int4_us": t_kernel * 1e6, "int4_hadamard_us": t_had * 1e6,
                           "speedup_int4": t_base / t_kernel, "speedup_int4_hadamard": t_base / t_had,
                           "int4_hadamard_tops": 2.0 * m * n * k / t_had / 1e12})
         del weight, wp
@@ -1011,7 +1008,7 @@ def run_sweep(args):
             x = torch.randn(m, 4096, generator=g, device=dev).to(torch.bfloat16)
             sc = torch.empty(m, 1, dtype=torch.bfloat16, device=dev)
             rs = torch.empty(m, 1, dtype=torch.int32, device=dev)
-            a8 = quest.prefers_a8(m, 4096, n)  # the route linear_forward takes for this shape
+            a8 = quest.prefers_a8(m, 4096, n)  # what the two ops write and read between them
             code_bytes = m * (4096 if a8 else 2048)
             gemm_bytes = code_bytes + n * 2048 + 2.0 * m * n + 6.0 * (m + n)
             ns = sets_for(gemm_bytes)
@@ -1025,13 +1022,11 @@ def run_sweep(args):
             t_q = rotating_sets_time(lambda i: f1(sets[i][0], 128, sets[i][1], sc, rs), ns, reps, dev)
             t_g = rotating_sets_time(lambda i: mm(sets[i][1], sets[i][2], rs, wa, sc, ws, sets[i][3]), ns, reps, dev)
 
-            def both(i):  # the layer as linear_forward runs it (one library call, the GEMM launched behind the quantiser)
-                ws_kw = {"_a_int8": sets[i][1]} if a8 else {"_a_int_packed": sets[i][1]}
-                quest.linear_forward(sets[i][0], sets[i][2], ws, wa, out=sets[i][3], _a_scale=sc, _a_int_row_sum=rs,
-                                     use_hadamard=True, **ws_kw)
+            def both(i):  # the layer as linear_forward runs it: the library's route, one call
+                quest.linear_forward(sets[i][0], sets[i][2], ws, wa, out=sets[i][3], use_hadamard=True)
             t_l = rotating_sets_time(both, ns, reps, dev)
             ops = 2.0 * m * n * 4096
-            linear.append({"M": m, "N": n, "K": 4096, "route": "int8 operand" if a8 else "packed int4", "quantize_us": t_q * 1e6, "gemm_us": t_g * 1e6, "layer_us": t_l * 1e6,
+            linear.append({"M": m, "N": n, "K": 4096, "ops_operand": "int8" if a8 else "packed int4", "layer_route": layer_route(m, 4096, n), "quantize_us": t_q * 1e6, "gemm_us": t_g * 1e6, "layer_us": t_l * 1e6,
                            "gemm_tops": ops / t_g / 1e12, "gemm_frac_int8_peak": ops / t_g / 1e12 / (2 * peaks["bf16_tflops"]),
                            "gemm_gbs": gemm_bytes / t_g / 1e9, "gemm_frac_hbm": gemm_bytes / t_g / 1e9 / peaks["hbm_gbs"],
                            "layer_tops": ops / t_l / 1e12, "sets": ns})
