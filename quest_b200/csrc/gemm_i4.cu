@@ -1799,7 +1799,9 @@ extern "C" int quest_b200_layer_operand(int M, int K, int N) {
     // kernel needs several rounds (M 3 K 4096 N 11008 12.3 / 14.2, K 6400 N 9748 16.9 / 19.1, K 8192 N 10240 18.2 / 25.5);
     // never with a long K and few weight rows, which leave it too few warps (M 1 K 28672 N 1024: 20.4 / 14.8).
     if (gemv_eligible(M, K, N, 0) && (M <= 2 || (M <= 4 && ((long long)M * N * K <= 120000000ll || N >= 8192))) && !(K > 16384 && N < 4096)) return 0;
-    // A narrow layer on a large input pays for the operand's second byte: M 7008 K 28672 N 1024 261 against 271 us.
+    // A narrow layer on a large input pays for the operand's second byte (device time, packed / int8: M 7008 K 28672 N 1024 256 /
+    // 278 us, M 8192 K 11008 N 1024 141 / 143); with more columns the GEMM gains more than that (M 14127 K 7296 N 1344
+    // 195 / 174, M 65536 K 4096 N 1536 423 / 388, K = N = 8192 3707 / 2980).
     return (long long)M * K <= (48ll << 20) || N >= 1536;
 }
 

@@ -12,10 +12,9 @@
 //
 // What bounds it: the issue of the MMAs, then the power limit.  Four MMAs of 256 columns need 512 cycles of the tensor
 // pipe; issued from a `lane == 0` branch a 128-K step took 1250 cycles with .release.cluster arrivals, 700 with plain ones,
-// and takes 260 + 1.3 per column with the warp-uniform loop below.  Measured (GEMM alone, launches back to back), the
-// one-CTA 256 x 256 kernel on the same int8 operand against this one: M 2048 K 4096 N 4096 28.0 -> 24.5 us (2808 TOPS),
-// M 8192 K 4096 N 12288 305 -> 221 us (3723), M 2048 K 28672 N 8192 273-289 -> 258 us, M 512 K 4096 N 4096 29.1 -> 12.1 us,
-// M 1024 K 11008 N 4096 73 -> 31 us.
+// and takes 260 + 1.3 per column with the warp-uniform loop below.  Measured (GEMM alone, launches back to back, all operands
+// from HBM), the one-CTA 256 x 256 kernel on the same int8 operand against this one: K 4096, M 2048 N 4096 28.3 -> 26.3 us
+// (2609 TOPS), N 11008 74.0 -> 54.8, N 12288 78.9 -> 62.2; M 8192 N 4096 103 -> 79.5, N 12288 300 -> 225 (3670 TOPS).
 #pragma once
 
 namespace pair2 {
