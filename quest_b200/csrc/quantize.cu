@@ -334,7 +334,9 @@ __device__ __forceinline__ void silu8(const uint32_t (&w)[4], uint32_t (&t)[4]) 
     for (int i = 0; i < 4; ++i) t[i] = pack_bf16x2(q[2 * i], q[2 * i + 1]);
 }
 
-template <int HB, int UNITS, int PRO = kProNone>
+// A8: writes the GEMM's int8 operand (q_a8, K a multiple of 128) instead of packed codes.  A template parameter: as a run-time
+// test in the store loop it cost the packed form registers and 6 to 8 % (K 5632, 268 M elements, block 64: 185 -> 200 us).
+template <int HB, int UNITS, int PRO = kProNone, bool A8 = false>
 __global__ void __launch_bounds__(256, UNITS == 1 ? 4 : (UNITS == 2 ? 3 : 2))
 hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int nbuf) {
     extern __shared__ __align__(16) uint8_t hq_smem[];
@@ -541,8 +543,8 @@ hadamard_quant_mma_kernel(const RowParams p, const int W, const int G, const int
             const uint32_t out_base = smem_w + u * step_bytes + buf * kStepIn;  // input already consumed
             const uint4 w = quantise_unit(v[u], rc, out_base, lane, rs16);
             const int e0 = unit * kUnit + lane * 32;
-            if (row < M && p.q_a8 != nullptr) {  // K is a multiple of 128 here
-                if (e0 < K) store_a8(p.q_a8 + (size_t)row * K + e0, w);
+            if (A8) {
+                if (row < M && e0 < K) store_a8(p.q_a8 + (size_t)row * K + e0, w);
             } else if (row < M) {
                 uint8_t* dst = p.q_packed + (size_t)row * (K >> 1) + (e0 >> 1);
                 if (vec_store) {
@@ -616,8 +618,8 @@ static int launch_hq_mma(const RowParams& p_in, cudaStream_t stream) {
     }
     // Persistent grid: as many blocks as fit on the device at once (bounded by the number of row batches).
     // The caches are per kernel instantiation (index `which`) and per device.
-    static bool attr_done[3][64] = {{false}};
-    static int occ_cache[3][64][9][2] = {{{{0}}}};
+    static bool attr_done[6][64] = {{false}};
+    static int occ_cache[6][64][9][2] = {{{{0}}}};
     auto launch = [&](auto kernel, int which) -> int {
         const bool dev_ok = dev >= 0 && dev < 64;
         if (!(dev_ok && attr_done[which][dev])) {
@@ -654,6 +656,11 @@ static int launch_hq_mma(const RowParams& p_in, cudaStream_t stream) {
         }
         return launch_status();
     };
+    if (p.q_a8 != nullptr) {
+        if (per == 1) return launch(hadamard_quant_mma_kernel<HB, 1, PRO, true>, 3);
+        if (per == 2) return launch(hadamard_quant_mma_kernel<HB, 2, PRO, true>, 4);
+        return launch(hadamard_quant_mma_kernel<HB, 4, PRO, true>, 5);
+    }
     if (per == 1) return launch(hadamard_quant_mma_kernel<HB, 1, PRO>, 0);
     if (per == 2) return launch(hadamard_quant_mma_kernel<HB, 2, PRO>, 1);
     return launch(hadamard_quant_mma_kernel<HB, 4, PRO>, 2);
